@@ -141,8 +141,11 @@ __global__ void to_fp32_kernel(int64_t n, const double2 *__restrict__ src, float
 // ----------------------------------------------------------------------------
 // LDL^T factor (advlas_skyline_ldl_decomposite, advlas_skyline.c:79-128),
 // row-Crout without pivoting, in place: off-diagonals become L (unit lower),
-// the diagonal becomes 1/d.  One warp per subdomain; the dot products of each
-// (i, j) step are split across the lanes.
+// the diagonal becomes 1/d.  The dot product of each (i, j) step is split
+// over 32 partial sums, k = k0 + l, k0 + l + 32, ..., which a butterfly adds
+// up; both kernels below sum in this order and give the same bits.
+//
+// One warp per subdomain, row by row: any size.
 __global__ void factor_kernel(int32_t nsub, const int32_t *__restrict__ sub_order, const int64_t *__restrict__ int_off,
                               const int32_t *__restrict__ env_lo, const int64_t *__restrict__ env_ptr,
                               double2 *L, int32_t *status) {
@@ -185,6 +188,116 @@ __global__ void factor_kernel(int32_t nsub, const int32_t *__restrict__ sub_orde
     __syncwarp();
   }
   if (lane == 0 && bad) atomicMax(status, 1);
+}
+
+// One CTA per subdomain, by blocks of kFB columns.  The row-by-row kernel above
+// is one chain of dot products per subdomain (C2: 9,800 of them, 20 ms on the
+// longest), bound by their latency.  Entry (i, j) needs only row i up to
+// column j - 1 and row j, so
+//   - the rows of the block itself are finished column by column: row j's
+//     pivot and scaling by one warp, then (i, j) of the block's other rows,
+//     one eight-lane group each;
+//   - every later row's entries in the block's columns follow, one group per
+//     row, with no barrier until the block is done.
+// An eight-lane group holds the 32 partial sums of a dot product four to a
+// lane: the butterfly's first two steps are then sums within a lane.  Rows
+// are read through L1; the pivots and the row table stay in shared memory.
+constexpr int kFB = 16;
+constexpr int kFactorThreads = 256;
+
+size_t factor_block_smem(int max_interior) { return (size_t)max_interior * 24; }
+
+__global__ void __launch_bounds__(kFactorThreads) factor_block_kernel(const int32_t *__restrict__ sub_order,
+                                                                     const int64_t *__restrict__ int_off,
+                                                                     const int32_t *__restrict__ env_lo,
+                                                                     const int64_t *__restrict__ env_ptr, double2 *L,
+                                                                     int32_t *status) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int s = sub_order[blockIdx.x];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, j8 = lane & 7;
+  constexpr int kGroups = kFactorThreads / 8;
+  const int64_t o = int_off[s];
+  const int nI = (int)(int_off[s + 1] - o);
+  if (nI == 0) return;
+  double2 *dinv = (double2 *)smem_raw;  // pivots 1/d
+  int32_t *lo = (int32_t *)(dinv + nI);
+  int32_t *pr = lo + nI;                // row start less its first column: entry (i, k) at pr[i] + k
+  const int64_t base = env_ptr[o];
+  double2 *B = L + base;
+  for (int i = tid; i < nI; i += kFactorThreads) {
+    lo[i] = env_lo[o + i];
+    pr[i] = (int32_t)(env_ptr[o + i] - base) - lo[i];
+  }
+  __syncthreads();
+  // sum over k of (i, k) (j, k), the same value in the group's lanes (0 when
+  // the group has no entry); every lane of the warp calls it
+  auto dot = [&](bool act, int i, int j) {
+    double2 p[4] = {cz(), cz(), cz(), cz()};
+    if (act) {
+      const int k0 = max(lo[i], lo[j]);
+      const double2 *gi = B + pr[i], *lj = B + pr[j];
+      int k = k0 + j8;
+      for (; k + 24 < j; k += 32) {
+#pragma unroll
+        for (int u = 0; u < 4; u++) p[u] = cadd(p[u], cmul_rn(gi[k + 8 * u], lj[k + 8 * u]));
+      }
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        if (k + 8 * u < j) p[u] = cadd(p[u], cmul_rn(gi[k + 8 * u], lj[k + 8 * u]));
+    }
+    double2 v = cadd(cadd(p[0], p[2]), cadd(p[1], p[3]));
+#pragma unroll
+    for (int q = 4; q > 0; q >>= 1) v = cadd(v, shfl_xor(v, q));
+    return v;
+  };
+  bool bad = false;
+  for (int j0 = 0; j0 < nI; j0 += kFB) {
+    const int j1 = min(nI, j0 + kFB);
+    for (int j = j0; j < j1; j++) {
+      // row j: d = G_jj - sum G_jk^2 / d_k, and the scaled row
+      if (warp == 0) {
+        double2 *Gj = B + pr[j];
+        double2 acc = cz();
+        for (int k = lo[j] + lane; k < j; k += 32) {
+          const double2 g = Gj[k];
+          const double2 dk = dinv[k];
+          acc = cadd(acc, cmul_rn(cmul_rn(g, g), dk));
+          Gj[k] = cmul_rn(g, dk);
+        }
+        acc = warp_sum(acc);
+        if (lane == 0) {
+          const double2 d = csub(Gj[j], acc);
+          const double2 r = crecip_smith(d);
+          if (!(isfinite(r.x) && isfinite(r.y)) || ciszero(d)) bad = true;
+          Gj[j] = r;
+          dinv[j] = r;
+        }
+      }
+      __syncthreads();
+      // the block's later rows at column j
+      if (warp * 4 < j1 - j - 1) {
+        const int i = j + 1 + (tid >> 3);
+        const bool act = i < j1 && lo[min(i, nI - 1)] <= j;
+        const double2 v = dot(act, i, j);
+        if (act && j8 == 0) B[pr[i] + j] = csub(B[pr[i] + j], v);
+      }
+      __syncthreads();
+    }
+    // the rows below the block, at the block's columns
+    for (int i0 = j1 + warp * 4; i0 < nI; i0 += kGroups) {
+      const int i = i0 + (lane >> 3);
+      const bool row = i < nI && lo[min(i, nI - 1)] < j1;
+      if (!__any_sync(0xffffffffu, row)) continue;
+      for (int j = j0; j < j1; j++) {
+        const bool act = row && lo[min(i, nI - 1)] <= j;
+        const double2 v = dot(act, i, j);
+        if (act && j8 == 0) B[pr[i] + j] = csub(B[pr[i] + j], v);
+        __syncwarp();
+      }
+    }
+    __syncthreads();
+  }
+  if (bad) atomicMax(status, 1);
 }
 
 // ----------------------------------------------------------------------------
@@ -1593,6 +1706,14 @@ void launch_diag_pc(int64_t n, const int64_t *diag_src, const double2 *aval, dou
 
 void launch_factor(const DevProblem &p, const int64_t *int_off, const int32_t *env_lo, const int64_t *env_ptr,
                    double2 *L, int32_t *status, cudaStream_t stream) {
+  if (p.nsub <= 0) return;
+  // one CTA per subdomain while its row table fits in shared memory (9,600
+  // interior DOFs)
+  const size_t smem = factor_block_smem(p.max_interior);
+  if (raise_smem_limit((const void *)factor_block_kernel, kSlotFactor, smem) == 0) {
+    factor_block_kernel<<<p.nsub, kFactorThreads, smem, stream>>>(p.sub_order, int_off, env_lo, env_ptr, L, status);
+    return;
+  }
   factor_kernel<<<blocks_for((int64_t)p.nsub * 32, kThreads), kThreads, 0, stream>>>(p.nsub, p.sub_order, int_off,
                                                                                        env_lo, env_ptr, L, status);
 }

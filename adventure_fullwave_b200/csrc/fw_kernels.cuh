@@ -204,7 +204,7 @@ int configure_subsolve_inv(size_t smem, bool fp32);
 // envelope layout, in FP32 (Linv32) or FP64 (Linv64)
 void launch_inv_relayout(const DevProblem &p, const double2 *L64, bool fp32, cudaStream_t stream);
 // Raises (never lowers) the dynamic shared-memory limit of kernel `func` on
-// the current device; `slot` names the kernel (0..7).
+// the current device; `slot` names the kernel.
 // Slots of the process-wide dynamic shared-memory limits (raise_smem_limit):
 // one per kernel instantiation that runs above the 48 KB default.
 enum SmemSlot {
@@ -216,7 +216,8 @@ enum SmemSlot {
   kSlotInv64 = 5,
   kSlotMulti32 = 6,
   kSlotMulti64 = 7,
-  kSmemSlots = 8
+  kSlotFactor = 8,
+  kSmemSlots = 9
 };
 int raise_smem_limit(const void *func, int slot, size_t smem);
 // kernels one launch_subsolve call issues
