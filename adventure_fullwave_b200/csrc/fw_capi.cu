@@ -1307,13 +1307,6 @@ static int multi_setup(fwgpu_context *c) {
   if (fp32) {
     FW_TRY(c->alloc(&m.B, nI * R));
     FW_TRY(c->alloc(&m.Rres, nI * R));
-    float2 *z = nullptr;
-    FW_TRY(c->alloc(&z, nI * R));
-    m.Zs = z;
-  } else {
-    double2 *z = nullptr;
-    FW_TRY(c->alloc(&z, nI * R));
-    m.Zs = z;
   }
   FW_TRY(c->alloc(&m.P, nf * R));
   FW_TRY(c->alloc(&m.Q, nf * R));

@@ -25,11 +25,15 @@ __device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
   return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
-// a b with its roundings spelled out: the contraction that the compiler gives
-// cmul in the row-by-row kernels.  Kernels that must give the same bits as
-// those use this form, which no surrounding code can change.
+// a b with its roundings spelled out (re: a.x b.x fused, im: a.y b.x fused):
+// where a kernel must give the bits of another one, both of its products are
+// in this form or in the one with a and b exchanged, whichever contraction
+// the compiler chose there, and no surrounding code can change it.
 __device__ __forceinline__ double2 cmul_rn(double2 a, double2 b) {
   return make_double2(__fma_rn(a.x, b.x, -__dmul_rn(a.y, b.y)), __fma_rn(a.y, b.x, __dmul_rn(a.x, b.y)));
+}
+__device__ __forceinline__ float2 cmul_rn(float2 a, float2 b) {
+  return make_float2(__fmaf_rn(a.x, b.x, -__fmul_rn(a.y, b.y)), __fmaf_rn(a.y, b.x, __fmul_rn(a.x, b.y)));
 }
 // acc + a b and acc - a b as four fused multiply-adds into the accumulator
 // (the sweeps' inner products: two FP64 instructions fewer per entry than

@@ -151,7 +151,6 @@ struct MultiProblem {
   const double2 *fI, *fG;       // [n_interior][kMaxRhs], [n_slots][kMaxRhs]
   double2 *Y;                   // [n_interior][kMaxRhs]: right-hand sides in, interior solutions out
   double2 *B, *Rres;            // FP32 + refinement: right-hand side copy, residual
-  void *Zs;                     // [n_interior][kMaxRhs] z stash in the factor's precision
   double2 *V, *qloc;            // [n_slots][kMaxRhs]
   double2 *P, *Q, *R, *Z, *U;   // [nfree][kMaxRhs]
   double2 *PC;                  // [nfree]

@@ -6,19 +6,17 @@
 // 16 values of one DOF are one 256-byte (FP64) line.  The subdomain phase of
 // an iteration is three launches, as in the single-source staged path:
 //   multi_rhs_kernel     f_I - A_IG v for every (interior row, source),
-//   multi_sweep_kernel   the envelope sweeps, 16/kRW warps per subdomain
-//                        with kRW sources each: lane groups take the kRW
-//                        sources and split every row's dot product; the
-//                        factor entries come from the TMA-staged row blocks
-//                        as shared-memory broadcasts, so one staged block
-//                        serves kRW sources and one row's dependent chain is
-//                        shared by all of them,
+//   multi_sweep_kernel   the envelope sweeps, one CTA per subdomain and
+//                        kRS sources; the factor entries come from the
+//                        TMA-staged row blocks as shared-memory broadcasts,
+//                        so one staged block serves kRS sources,
 //   multi_iface_kernel   q = A_G.[x; v] (- f_G) for every (slot, source).
 // The COCG kernels keep one set of scalars and a stopping status per source
 // (ITERATION_S, hddm_solver_s.h:260-400, per source); a finished source
 // keeps its vectors while the others go on.
 #include <cuda_runtime.h>
 
+#include <climits>
 #include <cstdint>
 #include <type_traits>
 
@@ -96,69 +94,77 @@ __global__ void multi_residual_kernel(MultiProblem m, int mode) {
 
 // ---- the sweeps --------------------------------------------------------------
 
+constexpr int kRS = 8;             // sources of one CTA
+constexpr int kSweepThreads = 256; // 32 rows (or columns) x kRS sources at a time
+
 struct MultiLayout {
-  size_t y, buf0, buf1, meta, rect, bar, blk, total;
+  size_t y, buf0, buf1, dinv, meta, rect, bar, blk, total;
 };
 
-__host__ __device__ inline MultiLayout multi_layout(int max_interior, int max_blocks, int cap, bool fp32, int rw) {
+__host__ __device__ inline MultiLayout multi_layout(int max_interior, int max_blocks, int cap, bool fp32) {
   const size_t es = fp32 ? 8 : 16;
   MultiLayout l;
   size_t o = 0;
   l.y = o;
-  o += a16((size_t)max_interior * rw * es);
+  o += a16((size_t)max_interior * kRS * es);
   l.buf0 = o;
   o += a16((size_t)cap * es);
   l.buf1 = o;
   o += a16((size_t)cap * es);
+  l.dinv = o;
+  o += a16((size_t)max_interior * es);
   l.meta = o;
   o += 32 * 8;
   l.rect = o;
-  o += a16((size_t)32 * rw * es);
+  o += a16((size_t)32 * kRS * es);
   l.bar = o;
-  o += 16;
+  o += 32;
   l.blk = o;
   o += a16(((size_t)max_blocks + 1) * 8);
   l.total = o;
   return l;
 }
 
-// Sources per sweep warp: 16 / kRW warps share a subdomain, each with kRW of
-// the 16 sources; lane = (group h, source r), kQ = 32 / kRW groups.  Per
-// staged block of rows r0 .. r0+nb-1:
-//   forward  - the entries left of the block for all its rows at once: group
-//              h takes rows h, h+kQ, ..., one accumulator per (row, source),
-//              the row's entries in order; no row waits for another.  Then
-//              the triangle row by row, y_i = b_i - (left_i + sum over the
-//              block's columns), the groups splitting the block's columns
-//              (shuffles add them), z_i = y_i / d_i;
-//   backward - the triangle row by row from the last: x_t final, then
-//              y_c -= L_tc x_t for the block's columns of row t; then the
-//              columns left of the block for all its rows: column c belongs to
-//              group c % kQ, which applies the rows from the last to the
-//              first in place, so no row waits for another.
-// Each (c, r) has one writer.  y holds the warp's kRW sources, [row][kRW].
-template <typename T, int kRW>
-__global__ void __launch_bounds__(32) multi_sweep_kernel(MultiProblem m, int mode, const double2 *rhs,
-                                                        double2 *xout, T *zstash, int accumulate, MultiLayout lay,
-                                                        int first) {
-  constexpr int kQ = 32 / kRW;
-  constexpr int kWarps = kR / kRW;
+// One CTA per (subdomain, kRS sources); the sources' vectors stay in shared
+// memory, y[row][kRS].  Per staged block of rows r0 .. r0+nb-1:
+//   forward  - the entries left of the block: thread (row, source) sums the
+//              row's entries in order, even and odd ones apart;
+//              then the triangle: one warp per source, lane t holding row t.
+//              A row's sum over the block's columns is split into kQ strands
+//              (column k0 + h, k0 + h + kQ, ...) of two alternating sums each,
+//              added pairwise: lane t keeps all 2 kQ of them and takes column
+//              j as soon as row j is final, so the strands cost no shuffle;
+//   backward - the triangle from the last row, one warp per source with lanes
+//              over columns; then the columns left of the block: thread
+//              (column, source) applies the block's rows from the last to the
+//              first in place.
+// The order of every sum is that of a row taken by kQ lane groups (FP64: 4,
+// FP32: 2), whatever the number of warps.  One warp for all the sources of a
+// subdomain, as before, left each row a chain of shuffles on one warp per
+// scheduler (16 sources on 551 subdomains of up to 600 elements: 1.97 ms per
+// iteration, FP32+IR on 83 of up to 1,000: 8.3 ms).
+template <typename T>
+__global__ void __launch_bounds__(kSweepThreads) multi_sweep_kernel(MultiProblem m, int mode, const double2 *rhs,
+                                                                   double2 *xout, int accumulate, MultiLayout lay,
+                                                                   int first) {
+  constexpr int kQ = sizeof(T) == 8 ? 2 : 4;
+  constexpr int kParts = kR / kRS;
+  constexpr int nt = kSweepThreads, nw = nt / 32;
   if (multi_stopped(m, mode)) return;
   const DevProblem &p = m.p;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int lane = threadIdx.x;
-  const int r = lane & (kRW - 1);
-  const int h = lane / kRW;
-  const int part = blockIdx.x % kWarps;  // which kRW sources
-  const int s = p.sub_order[first + blockIdx.x / kWarps];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int part = blockIdx.x % kParts;  // which kRS sources
+  const int s = p.sub_order[first + blockIdx.x / kParts];
   const int64_t io = p.int_off[s];
   const int nI = (int)(p.int_off[s + 1] - io);
   const int b0 = p.blk_off[s];
   const int nblk = p.blk_off[s + 1] - b0 - 1;
   if (nI == 0 || nblk <= 0) return;
   T *__restrict__ y = (T *)(smem_raw + lay.y);
+  T *__restrict__ dinv = (T *)(smem_raw + lay.dinv);
   int2 *meta = (int2 *)(smem_raw + lay.meta);
-  T *rect = (T *)(smem_raw + lay.rect);
+  T *__restrict__ rect = (T *)(smem_raw + lay.rect);
   int2 *blk = (int2 *)(smem_raw + lay.blk);
   Stage<T> st;
   st.buf0 = (T *)(smem_raw + lay.buf0);
@@ -168,129 +174,186 @@ __global__ void __launch_bounds__(32) multi_sweep_kernel(MultiProblem m, int mod
   stage_init(st, &m.ms->err, 0);
   const int64_t base = p.env_ptr[io];
   st.L = (sizeof(T) == 8 ? (const T *)(const void *)p.L32 : (const T *)(const void *)p.L64) + base;
-  for (int b = lane; b <= nblk; b += 32) blk[b] = p.blk_tab[b0 + b];
-  if (lane == 0) {
+  for (int b = tid; b <= nblk; b += nt) blk[b] = p.blk_tab[b0 + b];
+  if (tid == 0) {
     mbar_init(&st.bar[0], 1);
     mbar_init(&st.bar[1], 1);
     fence_mbar_init();
   }
-  // global vectors are [row][16]; this warp's sources are kRW*part ..
-  const int64_t g0 = io * kR + part * kRW;
-  for (int e = lane; e < nI * kRW; e += 32) y[e] = from_d2<T>(rhs[g0 + (int64_t)(e / kRW) * kR + (e % kRW)]);
-  __syncwarp();
+  // global vectors are [row][16]; this CTA's sources are kRS*part ..
+  const int64_t g0 = io * kR + part * kRS;
+  for (int e = tid; e < nI * kRS; e += nt) y[e] = from_d2<T>(rhs[g0 + (int64_t)(e / kRS) * kR + (e % kRS)]);
+  __syncthreads();
   const int32_t *lo_g = p.env_lo + io;
   const int64_t *ptr_g = p.env_ptr + io;
-  T *z = zstash + g0;
+  const int r = tid % kRS, row = tid / kRS;  // of the (row, source) passes
+  constexpr int kRows = nt / kRS;
 
   // forward
   bool ok = true;
   int nlo, npr;
-  stage_issue(st, 0, lane);
+  stage_issue(st, 0, tid);
   stage_row_meta(lo_g, ptr_g, base, blk[0].x, blk[1].x, lane, nlo, npr);
   for (int b = 0; b < nblk; b++) {
     const int r0 = blk[b].x, nb = blk[b + 1].x - r0;
-    meta[lane] = make_int2(nlo, npr);
+    const int my_lo = nlo, my_pr = npr;
+    if (warp == 0) meta[lane] = make_int2(nlo, npr);
     if (b + 1 < nblk) {
-      stage_issue(st, b + 1, lane);
+      stage_issue(st, b + 1, tid);
       stage_row_meta(lo_g, ptr_g, base, blk[b + 1].x, blk[b + 2].x, lane, nlo, npr);
     }
-    if (!__all_sync(0xffffffffu, stage_wait(st, b))) {
+    const bool late = !stage_wait(st, b);
+    if (__syncthreads_or(late)) {
       ok = false;
       break;
     }
-    __syncwarp();
     const T *S = ((b & 1) ? st.buf1 : st.buf0) - stage_a0(st, b);
-    // entries left of the block, every row of the block at once
-    for (int t = h; t < nb; t += kQ) {
+    // entries left of the block
+    for (int t = row; t < nb; t += kRows) {
       const int2 mt = meta[t];
       const int len = max(0, r0 - mt.x);
-      const T *__restrict__ row = S + mt.y;
-      const T *__restrict__ yk = y + (int64_t)mt.x * kRW + r;
+      const T *__restrict__ rw = S + mt.y;
+      const T *__restrict__ yk = y + mt.x * kRS + r;
       T a0 = czero<T>(), a1 = czero<T>();
       int k = 0;
-      for (; k + 1 < len; k += 2) {
-        a0 = cmac(a0, row[k], yk[k * kRW]);
-        a1 = cmac(a1, row[k + 1], yk[(k + 1) * kRW]);
-      }
-      if (k < len) a0 = cmac(a0, row[k], yk[k * kRW]);
-      rect[t * kRW + r] = cadd(a0, a1);
-    }
-    __syncwarp();
-    // the triangle, row by row over the block's columns
-    for (int t = 0; t < nb; t++) {
-      const int2 mt = meta[t];
-      const int i = r0 + t;
-      const int len = i - mt.x;
-      const int k0 = max(0, r0 - mt.x);
-      const T *__restrict__ row = S + mt.y;
-      const T *__restrict__ yk = y + (int64_t)mt.x * kRW + r;
-      T a0 = czero<T>(), a1 = czero<T>();
-      int k = k0 + h;
-      for (; k + kQ < len; k += 2 * kQ) {
-        a0 = cmac(a0, row[k], yk[k * kRW]);
-        a1 = cmac(a1, row[k + kQ], yk[(k + kQ) * kRW]);
-      }
-      if (k < len) a0 = cmac(a0, row[k], yk[k * kRW]);
-      T acc = cadd(a0, a1);
+      for (; k + 3 < len; k += 4) {
+        T w[4], v[4];
 #pragma unroll
-      for (int o = kRW; o < 32; o <<= 1) acc = cadd(acc, shfl_xor(acc, o));
-      const T val = csub(y[i * kRW + r], cadd(rect[t * kRW + r], acc));
-      const T dinv = row[len];
-      __syncwarp();
-      if (h == 0) {
-        y[i * kRW + r] = val;
-        z[(int64_t)i * kR + r] = cmul(val, dinv);
+        for (int u = 0; u < 4; u++) {
+          w[u] = rw[k + u];
+          v[u] = yk[(k + u) * kRS];
+        }
+        a0 = cmac(a0, w[0], v[0]);
+        a1 = cmac(a1, w[1], v[1]);
+        a0 = cmac(a0, w[2], v[2]);
+        a1 = cmac(a1, w[3], v[3]);
       }
-      __syncwarp();
+      for (; k < len; k += 2) {
+        a0 = cmac(a0, rw[k], yk[k * kRS]);
+        if (k + 1 < len) a1 = cmac(a1, rw[k + 1], yk[(k + 1) * kRS]);
+      }
+      rect[t * kRS + r] = cadd(a0, a1);
     }
+    __syncthreads();
+    // the triangle
+    for (int q = warp; q < kRS; q += nw) {
+      const bool in = lane < nb;
+      const T rc = in ? rect[lane * kRS + q] : czero<T>();
+      const T yv = in ? y[(r0 + lane) * kRS + q] : czero<T>();
+      const T *mine = S + my_pr - my_lo + r0;  // mine[j]: this lane's row at the block's column j
+      const int s0 = max(0, my_lo - r0);       // its first column in the block
+      // strand of column j: (j - s0) mod 2 kQ.  The sums are kept at j mod
+      // 2 kQ; which two strands are added first then depends on s0's parity
+      T a[2 * kQ];
+#pragma unroll
+      for (int u = 0; u < 2 * kQ; u++) a[u] = czero<T>();
+      T val = czero<T>();
+      for (int j0 = 0; j0 < nb; j0 += 2 * kQ) {
+        T op[2 * kQ];
+#pragma unroll
+        for (int u = 0; u < 2 * kQ; u++) op[u] = lane > j0 + u && in && j0 + u >= s0 ? mine[j0 + u] : czero<T>();
+#pragma unroll
+        for (int u = 0; u < 2 * kQ; u++) {
+          const int j = j0 + u;
+          if (j < nb) {
+            T h[kQ];
+#pragma unroll
+            for (int z = 0; z < kQ; z++) h[z] = cadd(a[z], a[z + kQ]);
+            T tot;
+            if (kQ == 2) {
+              tot = cadd(h[0], h[1]);
+            } else {
+              const bool odd = s0 & 1;
+              tot = cadd(cadd(h[0], odd ? h[3] : h[1]), cadd(h[2 % kQ], odd ? h[1] : h[3 % kQ]));
+            }
+            const T fin = csub(yv, cadd(rc, tot));
+            if (lane == j) val = fin;
+            const T yj = shfl_idx(fin, j);
+            if (lane > j && j >= s0) a[u] = cmac(a[u], op[u], yj);
+          }
+        }
+      }
+      if (in) {
+        y[(r0 + lane) * kRS + q] = val;
+        if (q == 0) dinv[r0 + lane] = mine[lane];  // 1/d on the diagonal
+      }
+    }
+    __syncthreads();
   }
-  for (int e = lane; e < nI * kRW; e += 32) y[e] = z[(int64_t)(e / kRW) * kR + (e % kRW)];
-  __syncwarp();
+  if (ok) {
+    for (int e = tid; e < nI * kRS; e += nt) y[e] = cmul_rn(dinv[e / kRS], y[e]);
+    __syncthreads();
+  }
 
   // backward
-  stage_row_meta(lo_g, ptr_g, base, blk[nblk - 1].x, blk[nblk].x, lane, nlo, npr);
+  if (ok) stage_row_meta(lo_g, ptr_g, base, blk[nblk - 1].x, blk[nblk].x, lane, nlo, npr);
   for (int b = nblk - 1; b >= 0 && ok; b--) {
     const int r0 = blk[b].x, nb = blk[b + 1].x - r0;
-    meta[lane] = make_int2(nlo, npr);
+    int bmin = lane < nb ? nlo : INT_MAX;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) bmin = min(bmin, __shfl_xor_sync(0xffffffffu, bmin, o));
+    if (warp == 0) meta[lane] = make_int2(nlo, npr);
+    // the forward sweep left blocks nblk-1 and nblk-2 in the buffers
     if (b >= 1) {
-      if (b - 1 < nblk - 2) stage_issue(st, b - 1, lane);
+      if (b - 1 < nblk - 2) stage_issue(st, b - 1, tid);
       stage_row_meta(lo_g, ptr_g, base, blk[b - 1].x, blk[b].x, lane, nlo, npr);
     }
-    if (!__all_sync(0xffffffffu, stage_wait(st, b))) {
+    const bool late = !stage_wait(st, b);
+    if (__syncthreads_or(late)) {
       ok = false;
       break;
     }
-    __syncwarp();
     const T *S = ((b & 1) ? st.buf1 : st.buf0) - stage_a0(st, b);
-    // the triangle from the last row: the block's columns of each row
-    for (int t = nb - 1; t >= 0; t--) {
-      const int2 mt = meta[t];
-      const int i = r0 + t;
-      const int len = i - mt.x;
-      const T xi = y[i * kRW + r];
-      const T *__restrict__ row = S + mt.y;
-      T *__restrict__ yc = y + (int64_t)mt.x * kRW + r;
-      for (int k = max(0, r0 - mt.x) + h; k < len; k += kQ) yc[k * kRW] = cmsub(yc[k * kRW], row[k], xi);
-      __syncwarp();
+    // the triangle from the last row, lanes over the block's columns
+    for (int q = warp; q < kRS; q += nw) {
+      T val = lane < nb ? y[(r0 + lane) * kRS + q] : czero<T>();
+      const int col = r0 + lane;
+      for (int i0 = nb - 1; i0 >= 1; i0 -= 4) {
+        T op[4];
+        bool act[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          const int i = i0 - u;
+          const int2 mt = meta[max(i, 0)];
+          act[u] = i >= 1 && lane < i && col >= mt.x;
+          op[u] = act[u] ? S[mt.y + col - mt.x] : czero<T>();
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          const T xi = shfl_idx(val, max(i0 - u, 0));
+          if (act[u]) val = cmsub(val, op[u], xi);
+        }
+      }
+      if (lane < nb) y[(r0 + lane) * kRS + q] = val;
     }
-    // the columns left of the block: column c belongs to group c % kQ, which
-    // applies the block's rows from the last to the first
-    for (int t = nb - 1; t >= 0; t--) {
-      const int2 mt = meta[t];
-      const int len = max(0, r0 - mt.x);
-      const T xi = y[(r0 + t) * kRW + r];
-      const T *__restrict__ row = S + mt.y;
-      T *__restrict__ yc = y + (int64_t)mt.x * kRW + r;
-      int k = (h - mt.x % kQ + kQ) % kQ;  // the first column of this group
-      for (; k < len; k += kQ) yc[k * kRW] = cmsub(yc[k * kRW], row[k], xi);
+    __syncthreads();
+    // the columns left of the block
+    for (int c = bmin + row; c < r0; c += kRows) {
+      T yc = y[c * kRS + r];
+      for (int t0 = nb - 1; t0 >= 0; t0 -= 4) {
+        T w[4], x[4];
+        bool act[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          const int t = max(t0 - u, 0);
+          const int2 mt = meta[t];
+          act[u] = t0 - u >= 0 && c >= mt.x;
+          w[u] = act[u] ? S[mt.y + c - mt.x] : czero<T>();
+          x[u] = y[(r0 + t) * kRS + r];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+          if (act[u]) yc = cmsub(yc, w[u], x[u]);
+      }
+      y[c * kRS + r] = yc;
     }
-    __syncwarp();
+    __syncthreads();
   }
   // every copy issued into this CTA's shared memory has landed before it exits
   stage_drain(st);
   if (!ok) return;
-  for (int e = lane; e < nI * kRW; e += 32) {
-    const int64_t ge = g0 + (int64_t)(e / kRW) * kR + (e % kRW);
+  for (int e = tid; e < nI * kRS; e += nt) {
+    const int64_t ge = g0 + (int64_t)(e / kRS) * kR + (e % kRS);
     double2 x = make_double2((double)y[e].x, (double)y[e].y);
     if (accumulate) x = cadd(xout[ge], x);
     xout[ge] = x;
@@ -534,23 +597,20 @@ unsigned grid_for(int64_t n, int threads) { return n > 0 ? (unsigned)((n + threa
 
 }  // namespace
 
-// sources per sweep warp: FP64 8 (its vectors are twice as large), FP32 16
-constexpr int kRwFp64 = 8, kRwFp32 = 16;
-
 size_t multi_smem_bytes(int max_interior, int max_blocks, int cap, bool fp32) {
-  return multi_layout(max_interior, max_blocks, cap, fp32, fp32 ? kRwFp32 : kRwFp64).total;
+  return multi_layout(max_interior, max_blocks, cap, fp32).total;
 }
 
 int configure_multi(size_t smem, bool fp32) {
-  return fp32 ? raise_smem_limit((const void *)multi_sweep_kernel<float2, kRwFp32>, kSlotMulti32, smem)
-              : raise_smem_limit((const void *)multi_sweep_kernel<double2, kRwFp64>, kSlotMulti64, smem);
+  return fp32 ? raise_smem_limit((const void *)multi_sweep_kernel<float2>, kSlotMulti32, smem)
+              : raise_smem_limit((const void *)multi_sweep_kernel<double2>, kSlotMulti64, smem);
 }
 
 // The sweep, one launch per size bucket, each with the shared memory of its
 // largest subdomain (a single bucket of every subdomain when none are set).
-template <typename T, int kRW>
+template <typename T>
 static void launch_multi_sweep(const MultiProblem &m, int mode, bool fp32, const double2 *rhs, double2 *xout,
-                               T *zstash, int accumulate, cudaStream_t stream) {
+                               int accumulate, cudaStream_t stream) {
   const DevProblem &p = m.p;
   const int nb = m.n_buckets > 0 ? m.n_buckets : 1;
   for (int k = 0; k < nb; k++) {
@@ -559,9 +619,9 @@ static void launch_multi_sweep(const MultiProblem &m, int mode, bool fp32, const
     const int mi = m.n_buckets > 0 ? m.bucket_max_interior[k] : p.max_interior;
     const int mb = m.n_buckets > 0 ? m.bucket_max_blocks[k] : p.max_blocks;
     if (count <= 0) continue;
-    const MultiLayout lay = multi_layout(mi, mb, p.stage_cap, fp32, kRW);
-    multi_sweep_kernel<T, kRW><<<(unsigned)count * (kR / kRW), 32, lay.total, stream>>>(m, mode, rhs, xout, zstash,
-                                                                                       accumulate, lay, first);
+    const MultiLayout lay = multi_layout(mi, mb, p.stage_cap, fp32);
+    multi_sweep_kernel<T><<<(unsigned)count * (kR / kRS), kSweepThreads, lay.total, stream>>>(m, mode, rhs, xout,
+                                                                                             accumulate, lay, first);
   }
 }
 
@@ -571,14 +631,13 @@ void launch_multi_subsolve(const MultiProblem &m, int mode, bool fp32, cudaStrea
   double2 *rhs = fp32 ? m.B : m.Y;
   multi_rhs_kernel<<<gi, 256, 0, stream>>>(m, mode, rhs);
   if (fp32) {
-    float2 *zs = (float2 *)m.Zs;
-    launch_multi_sweep<float2, kRwFp32>(m, mode, true, m.B, m.Y, zs, 0, stream);
+    launch_multi_sweep<float2>(m, mode, true, m.B, m.Y, 0, stream);
     for (int k = 0; k < p.ir_steps; k++) {
       multi_residual_kernel<<<gi, 256, 0, stream>>>(m, mode);
-      launch_multi_sweep<float2, kRwFp32>(m, mode, true, m.Rres, m.Y, zs, 1, stream);
+      launch_multi_sweep<float2>(m, mode, true, m.Rres, m.Y, 1, stream);
     }
   } else {
-    launch_multi_sweep<double2, kRwFp64>(m, mode, false, m.Y, m.Y, (double2 *)m.Zs, 0, stream);
+    launch_multi_sweep<double2>(m, mode, false, m.Y, m.Y, 0, stream);
   }
   multi_iface_kernel<<<gs, 256, 0, stream>>>(m, mode);
 }
