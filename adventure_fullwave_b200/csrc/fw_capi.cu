@@ -1320,23 +1320,29 @@ static int multi_setup(fwgpu_context *c) {
   return FWGPU_OK;
 }
 
-// Size buckets of the batched sweep: the subdomains in interior-size order,
-// a new bucket where the size falls below 0.6 of the bucket's largest, so a
-// warp's vectors of many right-hand sides take shared memory for its own size
-// class, not for the largest subdomain of the model.
+// Size buckets of the batched sweep: the subdomains in interior-size order, a
+// new bucket where the shared memory of a subdomain lets more CTAs onto an SM
+// than that of the bucket's largest (a bucket is a launch with a tail of its
+// own, so none is made for less).
 static void set_multi_buckets(fwgpu_context *c) {
   fw::MultiProblem &m = c->mp;
   const fw::Plan &p = c->p;
+  const bool fp32 = c->opts.precision == FWGPU_PREC_FP32_IR;
   const int n = (int)c->h_order.size();
   m.n_buckets = 0;
   int i = 0;
   while (i < n) {
     const int k = m.n_buckets;
     const int lead = p.subs[c->h_order[i]].nI;
-    int j = i, mb = 0;
+    int j = i, mb = 0, ctas = 0;
     const bool last = k == fw::kMaxBuckets - 1;
-    while (j < n && (last || p.subs[c->h_order[j]].nI * 10 >= lead * 6 || j == i)) {
-      mb = std::max(mb, c->h_nblk[c->h_order[j]]);
+    while (j < n) {
+      const int s = c->h_order[j];
+      const int fit = fw::multi_ctas_per_sm(fw::multi_smem_bytes(std::max(1, p.subs[s].nI), std::max(1, c->h_nblk[s]),
+                                                                 c->dp.stage_cap, fp32));
+      if (j == i) ctas = fit;
+      if (!last && fit > ctas) break;
+      mb = std::max(mb, c->h_nblk[s]);
       j++;
     }
     m.bucket_first[k] = i;

@@ -164,6 +164,7 @@ struct MultiProblem {
 };
 
 size_t multi_smem_bytes(int max_interior, int max_blocks, int cap, bool fp32);
+int multi_ctas_per_sm(size_t smem);  // sweep CTAs that fit one SM (at most 2: registers)
 int configure_multi(size_t smem, bool fp32);
 void launch_multi_subsolve(const MultiProblem &m, int mode, bool fp32, cudaStream_t stream);
 void launch_multi_set_status(MultiScalars *ms, double eps, int32_t max_loop, cudaStream_t stream);

@@ -16,6 +16,7 @@
 // keeps its vectors while the others go on.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <climits>
 #include <cstdint>
 #include <type_traits>
@@ -37,59 +38,92 @@ __device__ __forceinline__ bool multi_stopped(const MultiProblem &m, int mode) {
   return mode == kModeIter && m.ms->all_status != 0;
 }
 
-// ---- grid-wide products, one thread per (row, source) -----------------------
+// ---- grid-wide products, one thread per (row, two sources) -------------------
+// A row's entries and columns are the same for its 16 sources: with two of
+// them per thread half as many threads load and decode them.
+
+struct Pair {
+  double2 a, b;
+};
+__device__ __forceinline__ Pair load_pair(const double2 *p) { return {p[0], p[1]}; }
 
 __global__ void multi_rhs_kernel(MultiProblem m, int mode, double2 *__restrict__ out) {
   if (multi_stopped(m, mode)) return;
   const DevProblem &p = m.p;
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int r = (int)(t % kR);
-  const int64_t i = t / kR;
+  const int r = 2 * (int)(t % (kR / 2));
+  const int64_t i = t / (kR / 2);
   if (i >= p.n_interior) return;
   const int64_t row = p.row0 + i;
-  double2 acc = cz();
+  Pair acc = {cz(), cz()};
   if (mode != kModeFirst) {
     const int64_t q1 = p.cpl_rowptr[row + 1];
-    for (int64_t q = p.cpl_rowptr[row]; q < q1; q++)
-      acc = cadd(acc, cmul(p.cpl_val[q], m.P[(int64_t)p.cpl_gcol[q] * kR + r]));
+#pragma unroll 4
+    for (int64_t q = p.cpl_rowptr[row]; q < q1; q++) {
+      const double2 v = p.cpl_val[q];
+      const Pair x = load_pair(m.P + (int64_t)p.cpl_gcol[q] * kR + r);
+      acc.a = cadd(acc.a, cmul(v, x.a));
+      acc.b = cadd(acc.b, cmul(v, x.b));
+    }
   }
-  out[row * kR + r] = csub(mode != kModeIter ? m.fI[row * kR + r] : cz(), acc);
+  const Pair f = mode != kModeIter ? load_pair(m.fI + row * kR + r) : Pair{cz(), cz()};
+  out[row * kR + r] = csub(f.a, acc.a);
+  out[row * kR + r + 1] = csub(f.b, acc.b);
 }
 
 __global__ void multi_iface_kernel(MultiProblem m, int mode) {
   if (multi_stopped(m, mode)) return;
   const DevProblem &p = m.p;
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int r = (int)(t % kR);
-  const int64_t i = t / kR;
+  const int r = 2 * (int)(t % (kR / 2));
+  const int64_t i = t / (kR / 2);
   if (i >= p.n_slots) return;
   const int64_t slot = p.slot0 + i;
   const bool with_bc = mode != kModeFirst;
-  double2 acc = cz();
+  Pair acc = {cz(), cz()};
   const int64_t q1 = p.ifr_rowptr[slot + 1];
+#pragma unroll 4
   for (int64_t q = p.ifr_rowptr[slot]; q < q1; q++) {
     const int64_t g = p.ifr_gcol[q];
-    const double2 x = g >= 0 ? m.Y[g * kR + r] : (with_bc ? m.P[(-g - 1) * kR + r] : cz());
-    acc = cadd(acc, cmul(p.ifr_val[q], x));
+    const double2 v = p.ifr_val[q];
+    const Pair x = g >= 0 ? load_pair(m.Y + g * kR + r) : (with_bc ? load_pair(m.P + (-g - 1) * kR + r) : Pair{cz(), cz()});
+    acc.a = cadd(acc.a, cmul(v, x.a));
+    acc.b = cadd(acc.b, cmul(v, x.b));
   }
-  if (mode != kModeIter) acc = csub(acc, m.fG[slot * kR + r]);
-  m.qloc[slot * kR + r] = acc;
-  if (mode == kModeLast) m.V[slot * kR + r] = with_bc ? m.P[(int64_t)p.if_ln[slot] * kR + r] : cz();
+  if (mode != kModeIter) {
+    const Pair f = load_pair(m.fG + slot * kR + r);
+    acc.a = csub(acc.a, f.a);
+    acc.b = csub(acc.b, f.b);
+  }
+  m.qloc[slot * kR + r] = acc.a;
+  m.qloc[slot * kR + r + 1] = acc.b;
+  if (mode == kModeLast) {
+    const Pair v = with_bc ? load_pair(m.P + (int64_t)p.if_ln[slot] * kR + r) : Pair{cz(), cz()};
+    m.V[slot * kR + r] = v.a;
+    m.V[slot * kR + r + 1] = v.b;
+  }
 }
 
 __global__ void multi_residual_kernel(MultiProblem m, int mode) {
   if (multi_stopped(m, mode)) return;
   const DevProblem &p = m.p;
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int r = (int)(t % kR);
-  const int64_t i = t / kR;
+  const int r = 2 * (int)(t % (kR / 2));
+  const int64_t i = t / (kR / 2);
   if (i >= p.n_interior) return;
   const int64_t row = p.row0 + i;
-  double2 acc = cz();
+  Pair acc = {cz(), cz()};
   const int64_t q1 = p.aii_rowptr[row + 1];
-  for (int64_t q = p.aii_rowptr[row]; q < q1; q++)
-    acc = cadd(acc, cmul(p.aii_val[q], m.Y[(int64_t)p.aii_gcol[q] * kR + r]));
-  m.Rres[row * kR + r] = csub(m.B[row * kR + r], acc);
+#pragma unroll 4
+  for (int64_t q = p.aii_rowptr[row]; q < q1; q++) {
+    const double2 v = p.aii_val[q];
+    const Pair x = load_pair(m.Y + (int64_t)p.aii_gcol[q] * kR + r);
+    acc.a = cadd(acc.a, cmul(v, x.a));
+    acc.b = cadd(acc.b, cmul(v, x.b));
+  }
+  const Pair f = load_pair(m.B + row * kR + r);
+  m.Rres[row * kR + r] = csub(f.a, acc.a);
+  m.Rres[row * kR + r + 1] = csub(f.b, acc.b);
 }
 
 // ---- the sweeps --------------------------------------------------------------
@@ -144,7 +178,7 @@ __host__ __device__ inline MultiLayout multi_layout(int max_interior, int max_bl
 // scheduler (16 sources on 551 subdomains of up to 600 elements: 1.97 ms per
 // iteration, FP32+IR on 83 of up to 1,000: 8.3 ms).
 template <typename T>
-__global__ void __launch_bounds__(kSweepThreads) multi_sweep_kernel(MultiProblem m, int mode, const double2 *rhs,
+__global__ void __launch_bounds__(kSweepThreads, 2) multi_sweep_kernel(MultiProblem m, int mode, const double2 *rhs,
                                                                    double2 *xout, int accumulate, MultiLayout lay,
                                                                    int first) {
   constexpr int kQ = sizeof(T) == 8 ? 2 : 4;
@@ -244,9 +278,13 @@ __global__ void __launch_bounds__(kSweepThreads) multi_sweep_kernel(MultiProblem
       const int s0 = max(0, my_lo - r0);       // its first column in the block
       // strand of column j: (j - s0) mod 2 kQ.  The sums are kept at j mod
       // 2 kQ; which two strands are added first then depends on s0's parity
-      T a[2 * kQ];
+      T a[2 * kQ], h[kQ];  // strands, and each pair's sum
 #pragma unroll
       for (int u = 0; u < 2 * kQ; u++) a[u] = czero<T>();
+#pragma unroll
+      for (int u = 0; u < kQ; u++) h[u] = czero<T>();
+      T e0 = czero<T>(), e1 = czero<T>();  // the two pairs of pairs (kQ = 4): {0, 1} and {2, 3}, or {0, 3} and {2, 1}
+      const bool odd = s0 & 1;
       T val = czero<T>();
       for (int j0 = 0; j0 < nb; j0 += 2 * kQ) {
         T op[2 * kQ];
@@ -256,20 +294,34 @@ __global__ void __launch_bounds__(kSweepThreads) multi_sweep_kernel(MultiProblem
         for (int u = 0; u < 2 * kQ; u++) {
           const int j = j0 + u;
           if (j < nb) {
-            T h[kQ];
-#pragma unroll
-            for (int z = 0; z < kQ; z++) h[z] = cadd(a[z], a[z + kQ]);
-            T tot;
-            if (kQ == 2) {
-              tot = cadd(h[0], h[1]);
-            } else {
-              const bool odd = s0 & 1;
-              tot = cadd(cadd(h[0], odd ? h[3] : h[1]), cadd(h[2 % kQ], odd ? h[1] : h[3 % kQ]));
-            }
+            const T tot = kQ == 2 ? cadd(h[0], h[1]) : cadd(e0, e1);
             const T fin = csub(yv, cadd(rc, tot));
             if (lane == j) val = fin;
             const T yj = shfl_idx(fin, j);
-            if (lane > j && j >= s0) a[u] = cmac(a[u], op[u], yj);
+            if (lane > j && j >= s0) {
+              a[u] = cmac(a[u], op[u], yj);
+              constexpr int kH = kQ - 1;
+              h[u & kH] = cadd(a[u & kH], a[(u & kH) + kQ]);
+              if (kQ == 4) {
+                // only the sum that holds this strand changes
+                if ((u & kH) == 0) e0 = cadd(h[0], odd ? h[kQ - 1] : h[1]);
+                if ((u & kH) == 1) {
+                  const T v = cadd(h[1], odd ? h[2 % kQ] : h[0]);
+                  if (odd)
+                    e1 = v;
+                  else
+                    e0 = v;
+                }
+                if ((u & kH) == 2) e1 = cadd(h[2 % kQ], odd ? h[1] : h[kQ - 1]);
+                if ((u & kH) == 3) {
+                  const T v = cadd(h[kQ - 1], odd ? h[0] : h[2 % kQ]);
+                  if (odd)
+                    e0 = v;
+                  else
+                    e1 = v;
+                }
+              }
+            }
           }
         }
       }
@@ -289,6 +341,7 @@ __global__ void __launch_bounds__(kSweepThreads) multi_sweep_kernel(MultiProblem
   if (ok) stage_row_meta(lo_g, ptr_g, base, blk[nblk - 1].x, blk[nblk].x, lane, nlo, npr);
   for (int b = nblk - 1; b >= 0 && ok; b--) {
     const int r0 = blk[b].x, nb = blk[b + 1].x - r0;
+    const int my_lo = nlo;
     int bmin = lane < nb ? nlo : INT_MAX;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) bmin = min(bmin, __shfl_xor_sync(0xffffffffu, bmin, o));
@@ -327,25 +380,30 @@ __global__ void __launch_bounds__(kSweepThreads) multi_sweep_kernel(MultiProblem
       if (lane < nb) y[(r0 + lane) * kRS + q] = val;
     }
     __syncthreads();
-    // the columns left of the block
-    for (int c = bmin + row; c < r0; c += kRows) {
-      T yc = y[c * kRS + r];
-      for (int t0 = nb - 1; t0 >= 0; t0 -= 4) {
+    // the columns left of the block: a warp's four columns take the rows that
+    // reach them, from the last
+    for (int cb = bmin + warp * (32 / kRS); cb < r0; cb += kRows) {
+      const int c = cb + lane / kRS;
+      uint32_t rows = __ballot_sync(0xffffffffu, lane < nb && my_lo < cb + 32 / kRS);
+      const bool in = c < r0;
+      T yc = in ? y[c * kRS + r] : czero<T>();
+      while (rows) {
         T w[4], x[4];
         bool act[4];
 #pragma unroll
         for (int u = 0; u < 4; u++) {
-          const int t = max(t0 - u, 0);
+          const int t = rows ? 31 - __clz(rows) : 0;
           const int2 mt = meta[t];
-          act[u] = t0 - u >= 0 && c >= mt.x;
+          act[u] = rows && in && c >= mt.x;
           w[u] = act[u] ? S[mt.y + c - mt.x] : czero<T>();
           x[u] = y[(r0 + t) * kRS + r];
+          rows &= ~(1u << t);
         }
 #pragma unroll
         for (int u = 0; u < 4; u++)
           if (act[u]) yc = cmsub(yc, w[u], x[u]);
       }
-      y[c * kRS + r] = yc;
+      if (in) y[c * kRS + r] = yc;
     }
     __syncthreads();
   }
@@ -601,6 +659,8 @@ size_t multi_smem_bytes(int max_interior, int max_blocks, int cap, bool fp32) {
   return multi_layout(max_interior, max_blocks, cap, fp32).total;
 }
 
+int multi_ctas_per_sm(size_t smem) { return (int)std::min<size_t>(2, (227 * 1024) / (smem + 1024)); }
+
 int configure_multi(size_t smem, bool fp32) {
   return fp32 ? raise_smem_limit((const void *)multi_sweep_kernel<float2>, kSlotMulti32, smem)
               : raise_smem_limit((const void *)multi_sweep_kernel<double2>, kSlotMulti64, smem);
@@ -627,7 +687,7 @@ static void launch_multi_sweep(const MultiProblem &m, int mode, bool fp32, const
 
 void launch_multi_subsolve(const MultiProblem &m, int mode, bool fp32, cudaStream_t stream) {
   const DevProblem &p = m.p;
-  const unsigned gi = grid_for(p.n_interior * kR, 256), gs = grid_for(p.n_slots * kR, 256);
+  const unsigned gi = grid_for(p.n_interior * kR / 2, 256), gs = grid_for(p.n_slots * kR / 2, 256);
   double2 *rhs = fp32 ? m.B : m.Y;
   multi_rhs_kernel<<<gi, 256, 0, stream>>>(m, mode, rhs);
   if (fp32) {
