@@ -79,7 +79,9 @@ struct fwgpu_context {
   int32_t *d_env_lo = nullptr;
   int64_t *d_env_ptr = nullptr;
   // operators and right-hand sides
-  std::vector<double2> h_b_local;  // TMP_B per local DOF (concatenated)
+  std::vector<fw::RhsPoint> h_points;  // the point source's entries of TMP_B, one per local DOF
+  fw::RhsPoint *d_points = nullptr;
+  size_t points_cap = 0;
   double2 *d_cpl_val = nullptr, *d_ifr_val = nullptr, *d_aii_val = nullptr, *d_pcloc = nullptr;
   double2 *d_fI = nullptr, *d_fG = nullptr;
   int64_t *d_edge_src = nullptr;
@@ -224,9 +226,8 @@ int build_rhs(fwgpu_context *c, const fwgpu_source *src) {
     return set_error(FWGPU_ERR_ARG, "a correction-Jo context takes its right-hand side from the antenna current");
   const fw::Plan &p = c->p;
   const int nsub = c->m.nsub;
-  std::vector<double2> fI(p.sub_int_off[nsub], make_double2(0.0, 0.0));
-  std::vector<double2> fG(p.sub_if_off[nsub], make_double2(0.0, 0.0));
-  c->h_b_local.assign(p.sub_dof_off[nsub], make_double2(0.0, 0.0));
+  const int64_t nI = p.sub_int_off[nsub], nG = p.sub_if_off[nsub];
+  std::vector<fw::RhsPoint> pts;
   if (src && src->n_entries > 0) {
     if (!src->edge || !src->value) return set_error(FWGPU_ERR_ARG, "source without edges or values");
     // owner subdomain and local DOF of every edge: the first subdomain holding it
@@ -245,45 +246,61 @@ int build_rhs(fwgpu_context *c, const fwgpu_source *src) {
         }
       }
     }
+    std::unordered_map<int64_t, size_t> seen;  // local DOF -> entry
     for (int k = 0; k < src->n_entries; k++) {
       const int e = src->edge[k];
       if (e < 0 || e >= c->m.ne) return set_error(FWGPU_ERR_ARG, "source edge out of range");
       const int s = owner[e], r = local[e];
       if (s < 0) continue;
-      const double2 val = make_double2(src->value[2 * k], src->value[2 * k + 1]);
-      double2 &b = c->h_b_local[p.sub_dof_off[s] + r];
-      b.x += val.x;
-      b.y += val.y;
-      const fw::SubHost &h = p.subs[s];
-      if (h.cidx[r] >= 0) {
-        fI[p.sub_int_off[s] + h.cidx[r]] = b;
-      } else if (h.slot[r] >= 0) {
-        fG[p.sub_if_off[s] + h.slot[r]] = b;
+      const int64_t dof = p.sub_dof_off[s] + r;
+      const auto at = seen.emplace(dof, pts.size());
+      if (at.second) {
+        const fw::SubHost &h = p.subs[s];
+        const int64_t to = h.cidx[r] >= 0   ? p.sub_int_off[s] + h.cidx[r]
+                           : h.slot[r] >= 0 ? -(p.sub_if_off[s] + h.slot[r]) - 2
+                                            : -1;
+        pts.push_back(fw::RhsPoint{dof, to, 0.0, 0.0});
       }
+      // values on one edge add up in their order
+      fw::RhsPoint &b = pts[at.first->second];
+      b.re += src->value[2 * k];
+      b.im += src->value[2 * k + 1];
     }
   }
+  c->h_points.swap(pts);
+  const size_t np = c->h_points.size();
   if (!c->d_fI) {
-    FW_TRY(c->alloc(&c->d_fI, fI.size()));
-    FW_TRY(c->alloc(&c->d_fG, fG.size()));
+    FW_TRY(c->alloc(&c->d_fI, nI));
+    FW_TRY(c->alloc(&c->d_fG, nG));
   }
-  if (!fI.empty())
-    FW_CUDA(cudaMemcpyAsync(c->d_fI, fI.data(), fI.size() * sizeof(double2), cudaMemcpyHostToDevice, c->stream));
-  if (!fG.empty())
-    FW_CUDA(cudaMemcpyAsync(c->d_fG, fG.data(), fG.size() * sizeof(double2), cudaMemcpyHostToDevice, c->stream));
-  if (c->el_src && !c->el_src_off) {
+  if (np > c->points_cap) {
+    c->release(c->d_points);
+    c->d_points = nullptr;
+    c->points_cap = 0;
+    FW_TRY(c->alloc(&c->d_points, np));
+    c->points_cap = np;
+  }
+  const bool elements = c->el_src && !c->el_src_off;
+  const int64_t ndof = p.sub_dof_off[nsub];
+  if (elements && !c->d_b_local) {
+    FW_TRY(c->alloc(&c->d_b_local, ndof));
+    FW_TRY(c->alloc(&c->d_b_edge, ndof));
+  }
+  FW_CUDA(cudaMemsetAsync(c->d_fI, 0, nI * sizeof(double2), c->stream));
+  FW_CUDA(cudaMemsetAsync(c->d_fG, 0, nG * sizeof(double2), c->stream));
+  if (elements) FW_CUDA(cudaMemsetAsync(c->d_b_edge, 0, ndof * sizeof(double2), c->stream));
+  if (np > 0) {
+    FW_CUDA(cudaMemcpyAsync(c->d_points, c->h_points.data(), np * sizeof(fw::RhsPoint), cudaMemcpyHostToDevice,
+                            c->stream));
+    fw::launch_rhs_point((int32_t)np, c->d_points, elements ? c->d_b_edge : nullptr, c->d_fI, c->d_fG, c->stream);
+    c->launches += 1;
+  }
+  if (elements) {
     // TMP_B = element contributions in element order, then the edge source;
     // the interior and interface right-hand sides are taken from it
-    const int64_t ndof = p.sub_dof_off[nsub];
-    if (!c->d_b_local) {
-      FW_TRY(c->alloc(&c->d_b_local, ndof));
-      FW_TRY(c->alloc(&c->d_b_edge, ndof));
-    }
-    if (ndof > 0)
-      FW_CUDA(cudaMemcpyAsync(c->d_b_edge, c->h_b_local.data(), ndof * sizeof(double2), cudaMemcpyHostToDevice,
-                              c->stream));
     fw::launch_rhs_gather(ndof, c->d_rhs_ptr, c->d_rhs_src, c->d_elrhs, c->d_b_edge, c->d_b_local, c->stream);
-    fw::launch_rhs_split((int64_t)fI.size(), c->d_int_pos, c->d_b_local, c->d_fI, c->stream);
-    fw::launch_rhs_split((int64_t)fG.size(), c->d_if_pos, c->d_b_local, c->d_fG, c->stream);
+    fw::launch_rhs_split(nI, c->d_int_pos, c->d_b_local, c->d_fI, c->stream);
+    fw::launch_rhs_split(nG, c->d_if_pos, c->d_b_local, c->d_fG, c->stream);
     c->launches += 3;
     FW_CUDA(cudaGetLastError());
   }
@@ -1382,12 +1399,9 @@ static int multi_run(fwgpu_context *c, int32_t n_src, const fwgpu_source *srcs, 
   FW_CUDA(cudaMemsetAsync((void *)m.fG, 0, nG * R * sizeof(double2), c->stream));
   for (int k = 0; k < n_src; k++) {
     FW_TRY(build_rhs(c, &srcs[k]));
-    if (nI > 0)
-      FW_CUDA(cudaMemcpy2DAsync((double2 *)m.fI + k, R * sizeof(double2), c->d_fI, sizeof(double2), sizeof(double2),
-                                nI, cudaMemcpyDeviceToDevice, c->stream));
-    if (nG > 0)
-      FW_CUDA(cudaMemcpy2DAsync((double2 *)m.fG + k, R * sizeof(double2), c->d_fG, sizeof(double2), sizeof(double2),
-                                nG, cudaMemcpyDeviceToDevice, c->stream));
+    fw::launch_multi_put(nI, k, c->d_fI, (double2 *)m.fI, c->stream);
+    fw::launch_multi_put(nG, k, c->d_fG, (double2 *)m.fG, c->stream);
+    c->launches += 2;
   }
   FW_CUDA(cudaEventRecord(c->ev[0], c->stream));
   FW_CUDA(cudaMemsetAsync(&m.ms->err, 0, sizeof(int32_t), c->stream));
@@ -1836,15 +1850,27 @@ int fwgpu_adjoint_gradient(fwgpu_context *c, int32_t n_probe, const int32_t *pro
   if (!c->d_xfwd) FW_TRY(c->alloc(&c->d_xfwd, ne));
   if (!c->d_te) FW_TRY(c->upload(&c->d_te, c->m.te));
   FW_CUDA(cudaMemcpyAsync(c->d_xfwd, c->d_xedge, ne * sizeof(double2), cudaMemcpyDeviceToDevice, c->stream));
-  std::vector<double2> xh(ne);
-  FW_CUDA(cudaMemcpyAsync(xh.data(), c->d_xedge, ne * sizeof(double2), cudaMemcpyDeviceToHost, c->stream));
-  FW_CUDA(cudaStreamSynchronize(c->stream));
+  // the probes' values alone come to the host
+  std::vector<double2> xh(n_probe);
+  if (n_probe > 0) {
+    std::vector<int64_t> at(probe_edges, probe_edges + n_probe);
+    int64_t *d_at = nullptr;
+    double2 *d_xp = nullptr;
+    FW_TRY(c->upload(&d_at, at));
+    FW_TRY(c->alloc(&d_xp, n_probe));
+    fw::launch_gather_ops(n_probe, d_at, c->d_xedge, d_xp, c->stream);
+    FW_CUDA(cudaGetLastError());
+    FW_CUDA(cudaMemcpyAsync(xh.data(), d_xp, n_probe * sizeof(double2), cudaMemcpyDeviceToHost, c->stream));
+    FW_CUDA(cudaStreamSynchronize(c->stream));
+    c->release(d_at);
+    c->release(d_xp);
+  }
   // J and the adjoint source dJ/dx = conj(x_P)
   double Jv = 0.0;
   std::vector<int32_t> pe(probe_edges, probe_edges + n_probe);
   std::vector<double> pv(2 * (size_t)n_probe);
   for (int k = 0; k < n_probe; k++) {
-    const double2 v = xh[pe[k]];
+    const double2 v = xh[k];
     Jv += v.x * v.x + v.y * v.y;
     pv[2 * k] = v.x;
     pv[2 * k + 1] = -v.y;
@@ -2094,7 +2120,10 @@ int fwgpu_get_tmp_aij(fwgpu_context *c, int32_t s, int32_t *nnz, int32_t *row_pt
   }
   *nnz = k;
   if (b) {
-    std::vector<double2> bl(c->h_b_local.begin() + p.sub_dof_off[s], c->h_b_local.begin() + p.sub_dof_off[s + 1]);
+    std::vector<double2> bl(h.nmp, make_double2(0.0, 0.0));
+    for (const fw::RhsPoint &q : c->h_points)
+      if (q.dof >= p.sub_dof_off[s] && q.dof < p.sub_dof_off[s + 1])
+        bl[q.dof - p.sub_dof_off[s]] = make_double2(q.re, q.im);
     if (c->el_src && c->d_b_local)
       FW_CUDA(cudaMemcpy(bl.data(), c->d_b_local + p.sub_dof_off[s], h.nmp * sizeof(double2), cudaMemcpyDeviceToHost));
     for (int r = 0; r < h.nmp; r++) {

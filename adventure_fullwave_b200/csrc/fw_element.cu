@@ -21,6 +21,8 @@
 
 #include <cstdint>
 
+#include "fw_rhs.h"
+
 namespace fw {
 
 __constant__ int c_tet_n[6][4] = {{0, 1, 2, 3}, {0, 2, 3, 1}, {0, 3, 1, 2}, {1, 2, 0, 3}, {1, 3, 2, 0}, {2, 3, 0, 1}};
@@ -576,6 +578,26 @@ __global__ void rhs_split_kernel(int64_t n, const int64_t *__restrict__ pos, con
                                  double2 *__restrict__ f) {
   const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k < n) f[k] = b[pos[k]];
+}
+
+// A point source's entries (one per DOF) into the zeroed right-hand sides:
+// its handful of values is all that crosses to the device, not the vectors.
+__global__ void rhs_point_kernel(int32_t n, const RhsPoint *__restrict__ pt, double2 *__restrict__ b_edge,
+                                 double2 *__restrict__ fI, double2 *__restrict__ fG) {
+  const int32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  const RhsPoint q = pt[k];
+  const double2 v = make_double2(q.re, q.im);
+  if (b_edge) b_edge[q.dof] = v;
+  if (q.to >= 0)
+    fI[q.to] = v;
+  else if (q.to < -1)
+    fG[-q.to - 2] = v;
+}
+
+void launch_rhs_point(int32_t n, const RhsPoint *pt, double2 *b_edge, double2 *fI, double2 *fG, cudaStream_t stream) {
+  if (n <= 0) return;
+  rhs_point_kernel<<<(unsigned)((n + 127) / 128), 128, 0, stream>>>(n, pt, b_edge, fI, fG);
 }
 
 void launch_element_rhs(int64_t n_el, const int32_t *el_order, const int32_t *tet_vertices, const double *crd,

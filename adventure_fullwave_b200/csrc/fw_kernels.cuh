@@ -5,6 +5,8 @@
 
 #include <cstdint>
 
+#include "fw_rhs.h"
+
 namespace fw {
 
 // COCG scalars of one interface problem, resident on the device.  Mirrors the
@@ -170,6 +172,8 @@ void launch_multi_subsolve(const MultiProblem &m, int mode, bool fp32, cudaStrea
 void launch_multi_set_status(MultiScalars *ms, double eps, int32_t max_loop, cudaStream_t stream);
 void launch_multi_first(const MultiProblem &m, const double2 *pcloc, cudaStream_t stream);
 void launch_multi_iteration(const MultiProblem &m, bool fp32, cudaStream_t stream);
+// column k of the [n][kMaxRhs] vector dst = src
+void launch_multi_put(int64_t n, int k, const double2 *src, double2 *dst, cudaStream_t stream);
 void launch_multi_edge_solution(const MultiProblem &m, int k, int64_t ne, const int64_t *edge_src, double2 *x,
                                 cudaStream_t stream);
 int multi_iteration_launches(bool fp32, int ir_steps, int n_buckets);
@@ -235,6 +239,7 @@ void launch_element_rhs(int64_t n_el, const int32_t *el_order, const int32_t *te
                         double2 *be, cudaStream_t stream);
 void launch_rhs_gather(int64_t n_dof, const int64_t *ptr, const int32_t *src, const double2 *be,
                        const double2 *b_edge, double2 *b, cudaStream_t stream);
+void launch_rhs_point(int32_t n, const RhsPoint *pt, double2 *b_edge, double2 *fI, double2 *fG, cudaStream_t stream);
 void launch_rhs_split(int64_t n, const int64_t *pos, const double2 *b, double2 *f, cudaStream_t stream);
 void launch_post_em_E(int64_t nt, const int32_t *tet_vertices, const int32_t *tet_edges, const double *crd,
                       const uint8_t *el_has_nu, const double *el_sigma, double omega, const double2 *x, double2 *B,

@@ -651,6 +651,11 @@ __global__ void multi_edge_solution_kernel(int64_t ne, int k, const int64_t *__r
   x[e] = s >= 0 ? Y[s * kR + k] : (s < -1 ? V[(-s - 2) * kR + k] : make_double2(0.0, 0.0));
 }
 
+__global__ void multi_put_kernel(int64_t n, int k, const double2 *__restrict__ src, double2 *__restrict__ dst) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) dst[i * kR + k] = src[i];
+}
+
 unsigned grid_for(int64_t n, int threads) { return n > 0 ? (unsigned)((n + threads - 1) / threads) : 1u; }
 
 }  // namespace
@@ -720,6 +725,11 @@ void launch_multi_iteration(const MultiProblem &m, bool fp32, cudaStream_t strea
   multi_pq_kernel<<<m.p.n_part_blocks, kMT, 0, stream>>>(m);
   multi_update_kernel<<<m.p.n_part_blocks, kMT, 0, stream>>>(m);
   multi_pupdate_kernel<<<m.p.n_part_blocks, kMT, 0, stream>>>(m);
+}
+
+void launch_multi_put(int64_t n, int k, const double2 *src, double2 *dst, cudaStream_t stream) {
+  if (n <= 0) return;
+  multi_put_kernel<<<grid_for(n, 256), 256, 0, stream>>>(n, k, src, dst);
 }
 
 void launch_multi_edge_solution(const MultiProblem &m, int k, int64_t ne, const int64_t *edge_src, double2 *x,

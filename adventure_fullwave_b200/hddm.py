@@ -268,9 +268,9 @@ class HddmSolver:
         return [self._result(r) for r in res]
 
     def edge_solution_multi(self, k: int) -> np.ndarray:
-        x = np.zeros(2 * self.n_edges, dtype=np.float64)
+        x = np.empty(self.n_edges, dtype=np.complex128)
         _lib.check(self._lib.fwgpu_get_edge_solution_multi(self._h, int(k), _ptr(x, ctypes.c_double)))
-        return x[0::2] + 1j * x[1::2]
+        return x
 
     def resolve(self, source, raise_not_converged: bool = False) -> HddmResult:
         src, keep = self._source(source)
@@ -413,9 +413,9 @@ class HddmSolver:
 
     # -- results -----------------------------------------------------------
     def edge_solution(self) -> np.ndarray:
-        x = np.zeros(2 * self.n_edges, dtype=np.float64)
+        x = np.empty(self.n_edges, dtype=np.complex128)
         _lib.check(self._lib.fwgpu_get_edge_solution(self._h, _ptr(x, ctypes.c_double)))
-        return x[0::2] + 1j * x[1::2]
+        return x
 
     def history(self) -> np.ndarray:
         n = ctypes.c_int32()
