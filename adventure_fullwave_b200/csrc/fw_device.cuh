@@ -114,6 +114,14 @@ __device__ __forceinline__ float2 from_d2<float2>(double2 a) {
 __host__ __device__ inline size_t a16(size_t b) { return (b + 15) & ~(size_t)15; }
 
 
+// A kernel of an iteration may be started while the one before it drains
+// (launch_chained): it waits here for that one's results, before it reads or
+// writes anything, and lets the one after it start in the same way.
+__device__ __forceinline__ void chain_begin() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 __device__ __forceinline__ uint32_t smem_u32(const void *ptr) { return (uint32_t)__cvta_generic_to_shared(ptr); }
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
@@ -199,6 +207,55 @@ __device__ inline double reduce_partials(const double *part, int nb, int f, bool
   return r;
 }
 
+
+// The same for N fields at once (field f a maximum where bit f of kMax is
+// set): one pass of shuffles and one barrier for all of them.  Field f's
+// result is valid in thread f.  sh: 33 N doubles.
+template <int N, unsigned kMax>
+__device__ __forceinline__ double block_reduce(double (&v)[N], double *sh) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+    for (int f = 0; f < N; f++) {
+      const double x = __shfl_xor_sync(0xffffffffu, v[f], o);
+      v[f] = (kMax >> f & 1) ? fmax(v[f], x) : v[f] + x;
+    }
+  }
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  __syncthreads();
+  if (lane == 0) {
+#pragma unroll
+    for (int f = 0; f < N; f++) sh[f * 32 + wid] = v[f];
+  }
+  __syncthreads();
+  double r = 0.0;
+  if (threadIdx.x < N) {
+    const bool is_max = kMax >> threadIdx.x & 1;
+    const double *s = sh + threadIdx.x * 32;
+    for (int i = 0; i < (int)(blockDim.x >> 5); i++) r = is_max ? fmax(r, s[i]) : r + s[i];
+  }
+  return r;
+}
+
+// reduce_partials for fields f0 .. f0 + N - 1: out[] in every thread
+template <int N, unsigned kMax>
+__device__ __forceinline__ void reduce_partials_n(const double *part, int nb, int f0, double *sh, double (&out)[N]) {
+  double v[N];
+#pragma unroll
+  for (int f = 0; f < N; f++) v[f] = 0.0;
+  for (int i = threadIdx.x; i < nb; i += blockDim.x) {
+#pragma unroll
+    for (int f = 0; f < N; f++) {
+      const double x = __ldcg(part + (f0 + f) * nb + i);  // written by other CTAs of this grid
+      v[f] = (kMax >> f & 1) ? fmax(v[f], x) : v[f] + x;
+    }
+  }
+  const double r = block_reduce<N, kMax>(v, sh);
+  if (threadIdx.x < N) sh[32 * N + threadIdx.x] = r;
+  __syncthreads();
+#pragma unroll
+  for (int f = 0; f < N; f++) out[f] = sh[32 * N + f];
+}
 
 // True in the last CTA of the grid to get here, after every CTA wrote its
 // partials; that CTA then reduces them in block order (deterministic) and

@@ -21,6 +21,7 @@
 
 #include "fw_device.cuh"
 #include "fw_kernels.cuh"
+#include "fw_launch.cuh"
 
 namespace fw {
 
@@ -1157,6 +1158,7 @@ __device__ __forceinline__ double2 group_sum(double2 v) {
 // rhs[g] = f_I[g] (first and last solves) - A_IG v (all but the first)
 template <int kL>
 __global__ void rhs_kernel(DevProblem p, int mode, double2 *__restrict__ out) {
+  chain_begin();
   if (mode == kModeIter && p.sc->status != 0) return;
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const bool in = t / kL < p.n_interior;
@@ -1176,6 +1178,7 @@ __global__ void rhs_kernel(DevProblem p, int mode, double2 *__restrict__ out) {
 // values and gathered operands), the rest of a long row in a loop.
 template <int kL>
 __global__ void iface_product_kernel(DevProblem p, int mode) {
+  chain_begin();
   if (mode == kModeIter && p.sc->status != 0) return;
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const bool in = t / kL < p.n_slots;
@@ -1236,11 +1239,25 @@ __global__ void ir_residual_kernel(DevProblem p, int mode) {
 constexpr int kRedThreads = 256;
 enum { kFPqRe = 0, kFPqIm, kFMax, kFRzRe, kFRzIm, kFL2, kNFields };
 
+// (a DOF has two or three slots: their places, then their values, are loaded
+// four at a time)
 __device__ __forceinline__ double2 gather_slots(const DevProblem &p, const double2 *v, int g) {
   double2 q = cz();
-  for (int t = p.gq_ptr[g]; t < p.gq_ptr[g + 1]; t++) {
-    const int64_t sl = p.gq_slot[t];
-    if (sl >= p.slot0 && sl < p.slot0 + p.n_slots) q = cadd(q, v[sl]);
+  const int t1 = p.gq_ptr[g + 1];
+  for (int t = p.gq_ptr[g]; t < t1; t += 4) {
+    int64_t sl[4];
+    double2 x[4];
+    bool in[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) sl[u] = p.gq_slot[min(t + u, t1 - 1)];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      in[u] = t + u < t1 && sl[u] >= p.slot0 && sl[u] < p.slot0 + p.n_slots;
+      x[u] = v[in[u] ? sl[u] : p.slot0];
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+      if (in[u]) q = cadd(q, x[u]);
   }
   return q;
 }
@@ -1312,27 +1329,26 @@ __global__ void cocg_first_scalars_kernel(DevProblem p) {
 // Q gathered over subdomains (hddm_solver_s.h:273 with COM_RES_SP), (p, q),
 // and in the last CTA -alpha = -(r, z) / (p, q)  (hddm_solver_s.h:282-295)
 __global__ void cocg_gather_pq_kernel(DevProblem p) {
+  chain_begin();
   if (p.sc->status != 0) return;
-  __shared__ double sh[40];
-  double re = 0.0, im = 0.0;
+  __shared__ double sh[33 * 2];
+  double v[2] = {0.0, 0.0};
   for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < p.nfree; g += gridDim.x * blockDim.x) {
     const double2 q = gather_q(p, g);
     p.Q[g] = q;
     const double2 t = cmul(p.P[g], q);
-    re += t.x;
-    im += t.y;
+    v[0] += t.x;
+    v[1] += t.y;
   }
   const int nb = p.n_part_blocks;
-  double r = block_sum(re, sh);
-  if (threadIdx.x == 0) p.part[kFPqRe * nb + blockIdx.x] = r;
-  r = block_sum(im, sh);
-  if (threadIdx.x == 0) p.part[kFPqIm * nb + blockIdx.x] = r;
+  const double r = block_reduce<2, 0>(v, sh);
+  if (threadIdx.x < 2) p.part[(kFPqRe + threadIdx.x) * nb + blockIdx.x] = r;
   if (!last_cta(&p.sc->ticket[0])) return;
-  const double pr = reduce_partials(p.part, nb, kFPqRe, false, sh);
-  const double pi = reduce_partials(p.part, nb, kFPqIm, false, sh);
+  double t[2];
+  reduce_partials_n<2, 0>(p.part, nb, kFPqRe, sh, t);
   if (threadIdx.x == 0) {
     CocgScalars *sc = p.sc;
-    const double2 pq = make_double2(pr, pi);
+    const double2 pq = make_double2(t[0], t[1]);
     if (cabs_ref(sc->rz) < kNearlyZero && cabs_ref(pq) < kNearlyZero) {
       sc->malpha = cz();
     } else {
@@ -1344,39 +1360,32 @@ __global__ void cocg_gather_pq_kernel(DevProblem p) {
 
 // u += -alpha p, r += -alpha q, max|r|, z = r pc, (r, z)  (hddm_solver_s.h:297-344)
 __global__ void cocg_update_kernel(DevProblem p) {
+  chain_begin();
   if (p.sc->status != 0) return;
-  __shared__ double sh[40];
+  __shared__ double sh[33 * 4];
   const double2 ma = p.sc->malpha;
-  double mx = 0.0, rzr = 0.0, rzi = 0.0, l2 = 0.0;
+  double v[4] = {0.0, 0.0, 0.0, 0.0};  // max|r|, (r, z), |r|^2
   for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < p.nfree; g += gridDim.x * blockDim.x) {
     p.U[g] = cadd(p.U[g], cmul(ma, p.P[g]));
     const double2 r = cadd(p.R[g], cmul(ma, p.Q[g]));
     p.R[g] = r;
-    mx = fmax(mx, cabs_ref(r));
+    v[0] = fmax(v[0], cabs_ref(r));
     const double2 z = cmul(r, p.PC[g]);
     p.Z[g] = z;
     const double2 rz = cmul(r, z);
-    rzr += rz.x;
-    rzi += rz.y;
-    l2 += r.x * r.x + r.y * r.y;
+    v[1] += rz.x;
+    v[2] += rz.y;
+    v[3] += r.x * r.x + r.y * r.y;
   }
   const int nb = p.n_part_blocks;
-  double r;
-  r = block_max(mx, sh);
-  if (threadIdx.x == 0) p.part[kFMax * nb + blockIdx.x] = r;
-  r = block_sum(rzr, sh);
-  if (threadIdx.x == 0) p.part[kFRzRe * nb + blockIdx.x] = r;
-  r = block_sum(rzi, sh);
-  if (threadIdx.x == 0) p.part[kFRzIm * nb + blockIdx.x] = r;
-  r = block_sum(l2, sh);
-  if (threadIdx.x == 0) p.part[kFL2 * nb + blockIdx.x] = r;
+  const double r = block_reduce<4, 1>(v, sh);
+  if (threadIdx.x < 4) p.part[(kFMax + threadIdx.x) * nb + blockIdx.x] = r;
   // last CTA: resi, beta = (r', z') / (r, z), convergence and loop count
   // (hddm_solver_s.h:318-379, hddm_solver.h:125-143)
   if (!last_cta(&p.sc->ticket[1])) return;
-  const double rmx = reduce_partials(p.part, nb, kFMax, true, sh);
-  const double rzr_t = reduce_partials(p.part, nb, kFRzRe, false, sh);
-  const double rzi_t = reduce_partials(p.part, nb, kFRzIm, false, sh);
-  const double l2_t = reduce_partials(p.part, nb, kFL2, false, sh);
+  double t[4];
+  reduce_partials_n<4, 1>(p.part, nb, kFMax, sh, t);
+  const double rmx = t[0], rzr_t = t[1], rzi_t = t[2], l2_t = t[3];
   if (threadIdx.x == 0) {
     CocgScalars *sc = p.sc;
     const double resi = rmx * sc->r0inv;
@@ -1409,6 +1418,7 @@ __global__ void cocg_update_kernel(DevProblem p) {
 // After the last iteration's p = u the last CTA marks the loop finished
 // (status 2), so that the iterations left in a graph launch do nothing.
 __global__ void cocg_pupdate_kernel(DevProblem p) {
+  chain_begin();
   const int st = p.sc->status;
   if (st == 2) return;
   const double2 be = p.sc->beta;
@@ -1735,18 +1745,15 @@ void launch_staged(const DevProblem &p, int mode, bool fp32, cudaStream_t stream
   // one thread per row for both products: their rows are short (a few to a
   // few tens of entries) and the loads of several entries in flight per
   // thread beat lanes sharing a row (timed with 1, 2, 4 and 8 lanes)
-  rhs_kernel<1><<<blocks_min1(p.n_interior, 256), 256, 0, stream>>>(p, mode, rhs);
+  launch_chained(rhs_kernel<1>, blocks_min1(p.n_interior, 256), 256, 0, stream, p, mode, rhs);
   if (fp32) {
-    subsolve_staged_kernel<float2, kInv><<<p.nsub, 32 * p.stage_warps, lay.total, stream>>>(p, mode, p.B, p.Y, p.Y32,
-                                                                                           0, lay);
+    subsolve_staged_kernel<float2, kInv><<<p.nsub, 32 * p.stage_warps, lay.total, stream>>>(p, mode, p.B, p.Y, p.Y32, 0, lay);
     for (int k = 0; k < p.ir_steps; k++) {
       ir_residual_kernel<4><<<blocks_min1(p.n_interior * 4, 256), 256, 0, stream>>>(p, mode);
-      subsolve_staged_kernel<float2, kInv><<<p.nsub, 32 * p.stage_warps, lay.total, stream>>>(p, mode, p.Rres, p.Y,
-                                                                                             p.Y32, 1, lay);
+      subsolve_staged_kernel<float2, kInv><<<p.nsub, 32 * p.stage_warps, lay.total, stream>>>(p, mode, p.Rres, p.Y, p.Y32, 1, lay);
     }
   } else {
-    subsolve_staged_kernel<double2, kInv><<<p.nsub, 32 * p.stage_warps, lay.total, stream>>>(p, mode, p.Y, p.Y, p.Y,
-                                                                                            0, lay);
+    subsolve_staged_kernel<double2, kInv><<<p.nsub, 32 * p.stage_warps, lay.total, stream>>>(p, mode, p.Y, p.Y, p.Y, 0, lay);
   }
   iface_product_kernel<1><<<blocks_min1(p.n_slots, 256), 256, 0, stream>>>(p, mode);
 }
@@ -1839,9 +1846,9 @@ void launch_cocg_first(const DevProblem &p, const double2 *pcloc, cudaStream_t s
 }
 
 void launch_cocg_update(const DevProblem &p, cudaStream_t stream) {
-  cocg_gather_pq_kernel<<<p.n_part_blocks, kRedThreads, 0, stream>>>(p);
-  cocg_update_kernel<<<p.n_part_blocks, kRedThreads, 0, stream>>>(p);
-  cocg_pupdate_kernel<<<p.n_part_blocks, kRedThreads, 0, stream>>>(p);
+  launch_chained(cocg_gather_pq_kernel, p.n_part_blocks, kRedThreads, 0, stream, p);
+  launch_chained(cocg_update_kernel, p.n_part_blocks, kRedThreads, 0, stream, p);
+  launch_chained(cocg_pupdate_kernel, p.n_part_blocks, kRedThreads, 0, stream, p);
 }
 
 void launch_cocg_iteration(const DevProblem &p, cudaStream_t stream) {

@@ -23,6 +23,7 @@
 
 #include "fw_device.cuh"
 #include "fw_kernels.cuh"
+#include "fw_launch.cuh"
 
 namespace fw {
 
@@ -48,6 +49,7 @@ struct Pair {
 __device__ __forceinline__ Pair load_pair(const double2 *p) { return {p[0], p[1]}; }
 
 __global__ void multi_rhs_kernel(MultiProblem m, int mode, double2 *__restrict__ out) {
+  chain_begin();
   if (multi_stopped(m, mode)) return;
   const DevProblem &p = m.p;
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -72,6 +74,7 @@ __global__ void multi_rhs_kernel(MultiProblem m, int mode, double2 *__restrict__
 }
 
 __global__ void multi_iface_kernel(MultiProblem m, int mode) {
+  chain_begin();
   if (multi_stopped(m, mode)) return;
   const DevProblem &p = m.p;
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -420,44 +423,59 @@ __global__ void __launch_bounds__(kSweepThreads, 2) multi_sweep_kernel(MultiProb
 
 // ---- COCG, one set of scalars per source ------------------------------------
 
-// per-source block reduction: thread (gi, r) = (threadIdx.x >> 4, & 15)
-__device__ __forceinline__ double block_sum_r(double v, double *sh, bool is_max) {
+// per-source block reductions of N fields (field f a maximum where bit f of
+// kMax is set): thread (gi, r) = (threadIdx.x >> 4, & 15) brings source r's
+// values; field gi's result is valid in the threads gi < N.  sh: N (kMT +
+// kMT / kR) doubles.
+template <int N, unsigned kMax>
+__device__ __forceinline__ double block_reduce_r(const double (&v)[N], double *sh) {
+  constexpr int kW = kMT / kR * (kR + 1);
   const int r = threadIdx.x & (kR - 1), gi = threadIdx.x >> 4;
   __syncthreads();
-  sh[gi * (kR + 1) + r] = v;
+#pragma unroll
+  for (int f = 0; f < N; f++) sh[f * kW + gi * (kR + 1) + r] = v[f];
   __syncthreads();
   double a = 0.0;
-  if (gi == 0) {
+  if (gi < N) {
+    const bool is_max = kMax >> gi & 1;
     for (int j = 0; j < kMT / kR; j++) {
-      const double x = sh[j * (kR + 1) + r];
+      const double x = sh[gi * kW + j * (kR + 1) + r];
       a = is_max ? fmax(a, x) : a + x;
     }
   }
-  return a;  // valid in threads gi == 0
+  return a;
 }
 
-__device__ __forceinline__ void write_part(const MultiProblem &m, int f, double v) {
-  if ((threadIdx.x >> 4) == 0)
-    m.part[((int64_t)f * m.p.n_part_blocks + blockIdx.x) * kR + (threadIdx.x & (kR - 1))] = v;
+// this CTA's partials of fields f0 .. f0 + N - 1
+template <int N, unsigned kMax>
+__device__ __forceinline__ void write_parts(const MultiProblem &m, int f0, const double (&v)[N], double *sh) {
+  const double a = block_reduce_r<N, kMax>(v, sh);
+  const int gi = threadIdx.x >> 4;
+  if (gi < N) m.part[((int64_t)(f0 + gi) * m.p.n_part_blocks + blockIdx.x) * kR + (threadIdx.x & (kR - 1))] = a;
 }
 
-// the last CTA: field f of source r over all blocks, blocks split over the 16
-// thread groups and combined in group order (fixed order)
-__device__ double reduce_part_r(const MultiProblem &m, int f, bool is_max, double *sh) {
+// the last CTA: the fields of source r over all blocks, blocks split over the
+// 16 thread groups and combined in group order (fixed order); out[] in every thread
+template <int N, unsigned kMax>
+__device__ __forceinline__ void reduce_parts(const MultiProblem &m, int f0, double *sh, double (&out)[N]) {
   const int r = threadIdx.x & (kR - 1), gi = threadIdx.x >> 4;
   const int nb = m.p.n_part_blocks;
-  double a = 0.0;
+  double a[N];
+#pragma unroll
+  for (int f = 0; f < N; f++) a[f] = 0.0;
   for (int j = gi; j < nb; j += kMT / kR) {
-    const double x = __ldcg(m.part + ((int64_t)f * nb + j) * kR + r);
-    a = is_max ? fmax(a, x) : a + x;
+#pragma unroll
+    for (int f = 0; f < N; f++) {
+      const double x = __ldcg(m.part + ((int64_t)(f0 + f) * nb + j) * kR + r);
+      a[f] = (kMax >> f & 1) ? fmax(a[f], x) : a[f] + x;
+    }
   }
-  const double t = block_sum_r(a, sh, is_max);
+  const double t = block_reduce_r<N, kMax>(a, sh);
   __syncthreads();
-  if (gi == 0) sh[kMT + r] = t;
+  if (gi < N) sh[gi * kR + r] = t;
   __syncthreads();
-  const double v = sh[kMT + r];
-  __syncthreads();
-  return v;
+#pragma unroll
+  for (int f = 0; f < N; f++) out[f] = sh[f * kR + r];
 }
 
 __device__ __forceinline__ double2 gather_slots_r(const DevProblem &p, const double2 *v, int g, int r) {
@@ -480,7 +498,7 @@ __global__ void multi_set_status_kernel(MultiScalars *ms, double eps, int32_t ma
 
 // first step of every source (hddm_solver_s.h:158-256): Q, PC, r = q, z, p, max|r|, (r, z)
 __global__ void multi_first_kernel(MultiProblem m, const double2 *__restrict__ pcloc) {
-  __shared__ double sh[kMT + kR + 32];
+  __shared__ double sh[4 * (kMT + kMT / kR)];
   const DevProblem &p = m.p;
   const int r = threadIdx.x & (kR - 1), gi = threadIdx.x >> 4;
   double mx = 0.0, rzr = 0.0, rzi = 0.0, l2 = 0.0;
@@ -503,15 +521,12 @@ __global__ void multi_first_kernel(MultiProblem m, const double2 *__restrict__ p
     rzi += rz.y;
     l2 += q.x * q.x + q.y * q.y;
   }
-  write_part(m, kMMax, block_sum_r(mx, sh, true));
-  write_part(m, kMRzRe, block_sum_r(rzr, sh, false));
-  write_part(m, kMRzIm, block_sum_r(rzi, sh, false));
-  write_part(m, kML2, block_sum_r(l2, sh, false));
+  const double part[4] = {mx, rzr, rzi, l2};
+  write_parts<4, 1>(m, kMMax, part, sh);
   if (!last_cta(&m.ms->ticket[0])) return;
-  const double vmx = reduce_part_r(m, kMMax, true, sh);
-  const double vrr = reduce_part_r(m, kMRzRe, false, sh);
-  const double vri = reduce_part_r(m, kMRzIm, false, sh);
-  const double vl2 = reduce_part_r(m, kML2, false, sh);
+  double all[4];
+  reduce_parts<4, 1>(m, kMMax, sh, all);
+  const double vmx = all[0], vrr = all[1], vri = all[2], vl2 = all[3];
   if (gi == 0) {
     CocgScalars &c = m.ms->s[r];
     c.norm0 = vmx;
@@ -531,8 +546,9 @@ __global__ void multi_first_kernel(MultiProblem m, const double2 *__restrict__ p
 
 // Q and (p, q); last CTA: -alpha per iterating source
 __global__ void multi_pq_kernel(MultiProblem m) {
+  chain_begin();
   if (m.ms->all_status != 0) return;
-  __shared__ double sh[kMT + kR + 32];
+  __shared__ double sh[2 * (kMT + kMT / kR)];
   const DevProblem &p = m.p;
   const int r = threadIdx.x & (kR - 1), gi = threadIdx.x >> 4;
   double re = 0.0, im = 0.0;
@@ -544,11 +560,12 @@ __global__ void multi_pq_kernel(MultiProblem m) {
     re += t.x;
     im += t.y;
   }
-  write_part(m, kMPqRe, block_sum_r(re, sh, false));
-  write_part(m, kMPqIm, block_sum_r(im, sh, false));
+  const double part[2] = {re, im};
+  write_parts<2, 0>(m, kMPqRe, part, sh);
   if (!last_cta(&m.ms->ticket[1])) return;
-  const double pr = reduce_part_r(m, kMPqRe, false, sh);
-  const double pi = reduce_part_r(m, kMPqIm, false, sh);
+  double all[2];
+  reduce_parts<2, 0>(m, kMPqRe, sh, all);
+  const double pr = all[0], pi = all[1];
   if (gi == 0) {
     CocgScalars &c = m.ms->s[r];
     if (c.status == 0) {
@@ -561,8 +578,9 @@ __global__ void multi_pq_kernel(MultiProblem m) {
 
 // u += -alpha p, r += -alpha q, z, max|r|, (r, z); last CTA: resi, beta, stopping
 __global__ void multi_update_kernel(MultiProblem m) {
+  chain_begin();
   if (m.ms->all_status != 0) return;
-  __shared__ double sh[kMT + kR + 32];
+  __shared__ double sh[4 * (kMT + kMT / kR)];
   const DevProblem &p = m.p;
   const int r = threadIdx.x & (kR - 1), gi = threadIdx.x >> 4;
   const bool live = m.ms->s[r].status == 0;
@@ -583,15 +601,12 @@ __global__ void multi_update_kernel(MultiProblem m) {
       l2 += rv.x * rv.x + rv.y * rv.y;
     }
   }
-  write_part(m, kMMax, block_sum_r(mx, sh, true));
-  write_part(m, kMRzRe, block_sum_r(rzr, sh, false));
-  write_part(m, kMRzIm, block_sum_r(rzi, sh, false));
-  write_part(m, kML2, block_sum_r(l2, sh, false));
+  const double part[4] = {mx, rzr, rzi, l2};
+  write_parts<4, 1>(m, kMMax, part, sh);
   if (!last_cta(&m.ms->ticket[2])) return;
-  const double vmx = reduce_part_r(m, kMMax, true, sh);
-  const double vrr = reduce_part_r(m, kMRzRe, false, sh);
-  const double vri = reduce_part_r(m, kMRzIm, false, sh);
-  const double vl2 = reduce_part_r(m, kML2, false, sh);
+  double all[4];
+  reduce_parts<4, 1>(m, kMMax, sh, all);
+  const double vmx = all[0], vrr = all[1], vri = all[2], vl2 = all[3];
   if (gi == 0) {
     CocgScalars &c = m.ms->s[r];
     if (c.status == 0) {
@@ -619,6 +634,7 @@ __global__ void multi_update_kernel(MultiProblem m) {
 // p = z + beta p, or p = u for a source that just stopped; last CTA marks
 // stopped sources finished and the batch finished when all are
 __global__ void multi_pupdate_kernel(MultiProblem m) {
+  chain_begin();
   if (m.ms->all_status != 0) return;
   const DevProblem &p = m.p;
   const int r = threadIdx.x & (kR - 1), gi = threadIdx.x >> 4;
@@ -694,7 +710,7 @@ void launch_multi_subsolve(const MultiProblem &m, int mode, bool fp32, cudaStrea
   const DevProblem &p = m.p;
   const unsigned gi = grid_for(p.n_interior * kR / 2, 256), gs = grid_for(p.n_slots * kR / 2, 256);
   double2 *rhs = fp32 ? m.B : m.Y;
-  multi_rhs_kernel<<<gi, 256, 0, stream>>>(m, mode, rhs);
+  launch_chained(multi_rhs_kernel, gi, 256, 0, stream, m, mode, rhs);
   if (fp32) {
     launch_multi_sweep<float2>(m, mode, true, m.B, m.Y, 0, stream);
     for (int k = 0; k < p.ir_steps; k++) {
@@ -722,9 +738,9 @@ void launch_multi_first(const MultiProblem &m, const double2 *pcloc, cudaStream_
 
 void launch_multi_iteration(const MultiProblem &m, bool fp32, cudaStream_t stream) {
   launch_multi_subsolve(m, kModeIter, fp32, stream);
-  multi_pq_kernel<<<m.p.n_part_blocks, kMT, 0, stream>>>(m);
-  multi_update_kernel<<<m.p.n_part_blocks, kMT, 0, stream>>>(m);
-  multi_pupdate_kernel<<<m.p.n_part_blocks, kMT, 0, stream>>>(m);
+  launch_chained(multi_pq_kernel, m.p.n_part_blocks, kMT, 0, stream, m);
+  launch_chained(multi_update_kernel, m.p.n_part_blocks, kMT, 0, stream, m);
+  launch_chained(multi_pupdate_kernel, m.p.n_part_blocks, kMT, 0, stream, m);
 }
 
 void launch_multi_put(int64_t n, int k, const double2 *src, double2 *dst, cudaStream_t stream) {
