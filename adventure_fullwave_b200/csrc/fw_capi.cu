@@ -1124,36 +1124,34 @@ static int setup_stage(fwgpu_context *c) {
 // same bits on every run: AUTO times only variants that sum in the same
 // order.  The staging capacity sets the row blocks, and with them the
 // order of the sums, so AUTO keeps the default capacity (a rule on the
-// model's envelope, setup_stage) and times one, two and four warps per
-// subdomain, which share out whole row groups and column chunks and so sum
-// alike.  With FP32 factors AUTO runs the block-inverse sweep (a rule, not
-// a timed choice), with FP64 factors the staged sweep.  The CTA kernel sums
-// in another order and runs only when asked for.  An explicit WARP choice
-// times the staging capacities too.
+// model's envelope, setup_stage) and times two and four warps per subdomain,
+// and four and eight with the next block's rows taken ahead, which share out
+// whole row groups and column chunks and so sum alike.  With FP32 factors AUTO
+// runs the block-inverse sweep (a rule, not a timed choice), with FP64 factors
+// the staged sweep.  The CTA kernel sums in another order and runs only when
+// asked for.  An explicit WARP choice times the staging capacities too.
 static int tune_solve_kernel(fwgpu_context *c) {
   const bool fp32 = c->opts.precision == FWGPU_PREC_FP32_IR;
   struct Cand {
-    int variant, cap, warps;
+    int variant, cap, warps, ahead;
   };
   std::vector<Cand> cand;
   const bool any = c->opts.solve_kernel == FWGPU_SOLVE_AUTO;
+  // every way of sharing out a sweep that the caller's stage_warps allows;
+  // AUTO leaves out one warp, which was never the fastest
+  auto sweeps = [&](int variant, int cap) {
+    for (int warps = 1; warps <= 8; warps *= 2)
+      for (int ahead = warps == 8 ? 1 : 0; ahead <= (warps >= 4 ? 1 : 0); ahead++)
+        if (c->opts.stage_warps == warps || (c->opts.stage_warps == 0 && !(any && warps == 1)))
+          cand.push_back({variant, cap, warps, ahead});
+  };
   // AUTO runs the block-inverse sweep where it built that layout (FP32 factors)
   const bool any_inv = any && c->inv_ok;
-  if (any && c->warp_ok && !any_inv) {
-    for (int warps = 1; warps <= 4; warps *= 2)
-      if (c->opts.stage_warps == 0 || c->opts.stage_warps == warps)
-        cand.push_back({fw::kSolveWarp, c->dp.stage_cap, warps});
-    if (cand.empty()) cand.push_back({fw::kSolveWarp, c->dp.stage_cap, c->opts.stage_warps});
-  }
+  if (any && c->warp_ok && !any_inv) sweeps(fw::kSolveWarp, c->dp.stage_cap);
   if (c->opts.solve_kernel == FWGPU_SOLVE_WARP && c->warp_ok)
-    for (int cap : c->stage_caps)
-      for (int warps = 1; warps <= 4; warps *= 2)
-        if (c->opts.stage_warps == 0 || c->opts.stage_warps == warps) cand.push_back({fw::kSolveWarp, cap, warps});
-  if (any && !c->warp_ok && c->dp.cta_smem > 0) cand.push_back({fw::kSolveCta, 0, 1});
-  if ((c->opts.solve_kernel == FWGPU_SOLVE_BLOCKINV || any_inv) && c->inv_ok)
-    for (int warps = 1; warps <= 4; warps *= 2)
-      if (c->opts.stage_warps == 0 || c->opts.stage_warps == warps)
-        cand.push_back({fw::kSolveInv, c->dp.inv_cap, warps});
+    for (int cap : c->stage_caps) sweeps(fw::kSolveWarp, cap);
+  if (any && !c->warp_ok && c->dp.cta_smem > 0) cand.push_back({fw::kSolveCta, 0, 1, 0});
+  if ((c->opts.solve_kernel == FWGPU_SOLVE_BLOCKINV || any_inv) && c->inv_ok) sweeps(fw::kSolveInv, c->dp.inv_cap);
   if (cand.empty()) {
     c->solve_tuned = true;
     return FWGPU_OK;
@@ -1163,6 +1161,7 @@ static int tune_solve_kernel(fwgpu_context *c) {
   for (const Cand &k : cand) {
     c->dp.solve_variant = k.variant;
     c->dp.stage_warps = k.warps;
+    c->dp.stage_ahead = k.ahead;
     if (k.variant == fw::kSolveWarp && c->dp.stage_cap != k.cap) FW_TRY(build_stage_blocks(c, k.cap, nullptr));
     fw::launch_subsolve(c->dp, fw::kModeFirst, fp32, c->stream);
     FW_CUDA(cudaEventRecord(c->ev[4], c->stream));
@@ -1179,6 +1178,7 @@ static int tune_solve_kernel(fwgpu_context *c) {
   }
   c->dp.solve_variant = pick.variant;
   c->dp.stage_warps = pick.warps;
+  c->dp.stage_ahead = pick.ahead;
   if (pick.variant == fw::kSolveWarp && c->dp.stage_cap != pick.cap) FW_TRY(build_stage_blocks(c, pick.cap, nullptr));
   c->solve_tuned = true;
   return FWGPU_OK;

@@ -716,23 +716,23 @@ __global__ void __launch_bounds__(kCtaThreads) subsolve_cta_kernel(DevProblem p,
 }
 
 // ----------------------------------------------------------------------------
-// Staged subdomain solve: one warp per subdomain, row blocks brought into
-// shared memory by TMA bulk copies.
+// Staged subdomain solve: one CTA of one to eight warps per subdomain, row
+// blocks brought into shared memory by TMA bulk copies.
 //
 // The iteration's subdomain work is split in three launches:
 //   rhs_kernel           f_I - A_IG v for every interior row of every
 //                        subdomain (SetBC, aij_matrix_func.h:60-136),
-//   subsolve_staged_kernel  the envelope substitutions, one warp per subdomain,
+//   subsolve_staged_kernel  the envelope substitutions, one CTA per subdomain,
 //   iface_product_kernel q = A_G.[x; v] (- f_G) for every interface slot.
 // The two products are grid-wide sparse products: every row of every
-// subdomain in parallel, a few lanes per row, coalesced.  The substitution
-// warp therefore only streams its factor.
+// subdomain in parallel.  The substitution CTA therefore only streams its
+// factor.
 //
 // A subdomain's rows are cut on the host into blocks of at most 32 rows whose
 // stored entries fit one staging buffer (blk_tab).  The block's entries are
 // contiguous in the envelope, so one cp.async.bulk copies the whole block
 // into shared memory, completing on an mbarrier; the copy of block b+1 is in
-// flight while block b is computed (two buffers per warp).  The backward sweep
+// flight while block b is computed (two buffers per CTA).  The backward sweep
 // starts on the two blocks the forward sweep left in the buffers.
 //   forward  - entries left of the block: eight lanes per row (conflict-free
 //              shared loads of the entry and of y[col]), four rows per step;
@@ -748,16 +748,16 @@ __global__ void __launch_bounds__(kCtaThreads) subsolve_cta_kernel(DevProblem p,
 // products with N (four independent sums per lane) instead of substitutions.
 // The arithmetic is the reference's row-oriented envelope substitution
 // (advlas_skyline.c:134-167) with the forward sums regrouped; the grouping
-// depends on the rows' entries and the block boundaries only, so one, two or
-// four warps per subdomain give the same bits.  The copies of the forward sweep
-// keep their lines in L2 (evict_last) for the backward sweep, whose copies
+// depends on the rows' entries and the block boundaries only, so one to
+// eight warps per subdomain, with rows taken ahead or not, give the same bits.
+// The copies of the forward sweep keep their lines in L2 (evict_last) for the backward sweep, whose copies
 // are the lines' last use (evict_first).  Every mbarrier wait is bounded: on
 // a timeout the CTA raises the error word, issues no further copy, waits for
 // the copies in flight and returns (the host reports the solve as failed).
 constexpr int kSB = 32;        // rows per block at most, one per lane
 
 struct StageLayout {
-  size_t y, buf0, buf1, xb, rb, meta, gmin, bar, blk, total;
+  size_t y, buf0, buf1, rb, meta, bar, blk, total;
 };
 
 // Shared-memory slice of one subdomain warp of the staged solve.
@@ -771,20 +771,131 @@ __host__ __device__ inline StageLayout stage_layout(int max_interior, int max_bl
   o += a16((size_t)cap * es);
   l.buf1 = o;
   o += a16((size_t)cap * es);
-  l.xb = o;
-  o += a16(kSB * es);
   l.rb = o;
-  o += a16(2 * kSB * es);
+  o += a16(2 * kSB * es);  // forward: row sums and a block's vector; backward: two blocks' solutions
   l.meta = o;
-  o += kSB * 8;
-  l.gmin = o;
-  o += 16;
+  o += 2 * kSB * 8;        // two blocks' row tables
   l.bar = o;
   o += 32;
   l.blk = o;
   o += a16(((size_t)max_blocks + 1) * 8);
   l.total = o;
   return l;
+}
+
+// A block's triangle, by warp 0: lane t holds row r0 + t, one broadcast
+// shuffle per row, the operands of 4 steps loaded ahead (block-inverse:
+// products with N).  The pivot scaling z = y/d goes to the z stash for the
+// backward sweep.
+template <typename T, bool kInv>
+__device__ __forceinline__ void forward_triangle(const T *S, int r0, int nb, const int2 *meta, T *y, T *zstash,
+                                                 T *rectb, int lane) {
+  if (kInv) {
+    // y_b = (I + N) v with v = y_b - (the sums left of the block): lane t
+    // sums N_tj v_j over j in four chunks of 8 columns, one accumulator
+    // per chunk, in ascending j; no chain from row to row
+    const int2 ml = meta[nb - 1];
+    const T *N = S + ml.y + max(0, r0 - ml.x);  // after the block's left parts
+    const T *Nr = N + ((lane * (lane - 1)) >> 1);
+    T *vb = rectb + kSB;
+    const T v = lane < nb ? csub(y[r0 + lane], rectb[lane]) : czero<T>();
+    vb[lane] = v;
+    __syncwarp();
+    T acc[4] = {czero<T>(), czero<T>(), czero<T>(), czero<T>()};
+#pragma unroll
+    for (int jj = 0; jj < 8; jj++) {
+#pragma unroll
+      for (int c = 0; c < 4; c++) {
+        const int j = 8 * c + jj;  // straight-line code: the loads go ahead of the sums
+        const T a = (j < lane && lane < nb) ? Nr[j] : czero<T>();
+        acc[c] = cmac(acc[c], a, vb[j]);
+      }
+    }
+    const T val = cadd(v, cadd(cadd(acc[0], acc[1]), cadd(acc[2], acc[3])));
+    if (lane < nb) {
+      y[r0 + lane] = val;
+      zstash[r0 + lane] = cmul(val, N[((nb * (nb - 1)) >> 1) + lane]);  // the pivots' 1/d after N
+    }
+  } else {
+    const int2 mt = meta[lane];
+    const int my_lo = mt.x;
+    const T rect = rectb[lane];
+    T val = lane < nb ? csub(y[r0 + lane], rect) : czero<T>();
+    const T *mine = S + mt.y - my_lo;  // mine[col]: this lane's row at column col
+    for (int j0 = 0; j0 < nb - 1; j0 += 4) {
+      T op[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const int jj = j0 + u;
+        op[u] = (lane > jj && r0 + jj >= my_lo) ? mine[r0 + jj] : czero<T>();
+      }
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const T yj = shfl_idx(val, min(j0 + u, 31));
+        val = cmsub(val, op[u], yj);
+      }
+    }
+    if (lane < nb) {
+      y[r0 + lane] = val;
+      zstash[r0 + lane] = cmul(val, mine[r0 + lane]);  // 1/d on the diagonal
+    }
+  }
+}
+
+// The backward triangle, by warp 0: x of the block to y and xb.
+template <typename T, bool kInv>
+__device__ __forceinline__ void backward_triangle(const T *S, int r0, int nb, const int2 *meta, T *y, T *xb, int lane) {
+  if (kInv) {
+    // x_b = (I + N)^T w with w = y_b: lane j sums N_tj w_t over t in four
+    // chunks of 8 rows, one accumulator per chunk, in ascending t
+    const int2 ml = meta[nb - 1];
+    const T *N = S + ml.y + max(0, r0 - ml.x);
+    const T wv = lane < nb ? y[r0 + lane] : czero<T>();
+    T acc[4] = {czero<T>(), czero<T>(), czero<T>(), czero<T>()};
+#pragma unroll
+    for (int tt = 0; tt < 8; tt++) {
+#pragma unroll
+      for (int c = 0; c < 4; c++) {
+        const int t = 8 * c + tt;
+        const T a = (lane < t && t < nb) ? N[((t * (t - 1)) >> 1) + lane] : czero<T>();
+        acc[c] = cmac(acc[c], a, y[r0 + min(t, nb - 1)]);
+      }
+    }
+    const T val = cadd(wv, cadd(cadd(acc[0], acc[1]), cadd(acc[2], acc[3])));
+    __syncwarp();  // every lane has read y_b before it is overwritten
+    if (lane < nb) {
+      y[r0 + lane] = val;
+      xb[lane] = val;
+    }
+  } else {
+    // lanes over the block's columns; operands of 4 steps loaded ahead
+    T val = lane < nb ? y[r0 + lane] : czero<T>();
+    const int col = r0 + lane;
+    for (int i0 = nb - 1; i0 >= 1; i0 -= 4) {
+      T op[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const int i = i0 - u;
+        const int2 mt = meta[max(i, 0)];
+        op[u] = (i >= 1 && lane < i && col >= mt.x) ? S[mt.y + col - mt.x] : czero<T>();
+      }
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const T xi = shfl_idx(val, max(i0 - u, 0));
+        val = cmsub(val, op[u], xi);
+      }
+    }
+    if (lane < nb) {
+      y[r0 + lane] = val;
+      xb[lane] = val;
+    }
+  }
+}
+
+// the staged block b, by envelope element
+template <typename T>
+__device__ __forceinline__ const T *stage_block(const Stage<T> &st, int b) {
+  return ((b & 1) ? st.buf1 : st.buf0) - stage_a0(st, b);
 }
 
 // Forward sweep over the row blocks.  Per block of nb <= 32 rows starting at
@@ -795,22 +906,19 @@ __host__ __device__ inline StageLayout stage_layout(int max_interior, int max_bl
 //     accumulator, and three shuffles add the eight lanes.  The sum of a row
 //     therefore depends on its entries alone, not on the staging capacity or
 //     the number of warps;
-//   - the block's triangle: lane t holds row r0 + t, one broadcast shuffle per
-//     row, the operands of 4 steps loaded ahead;
-//   - the pivot scaling z = y/d goes to the z stash for the backward sweep.
+//   - the block's triangle (forward_triangle).
 // Returns false when a staged copy did not arrive (error word raised); the
 // caller drains the copies in flight and stops.
 template <typename T, bool kInv>
 __device__ bool staged_forward(Stage<T> &st, int nblk, const int32_t *lo_g, const int64_t *ptr_g, int64_t base,
-                               T *y, int2 *meta, T *zstash, T *rectb, int tid, int nw) {
-  const int lane = tid & 31, w = tid >> 5;
+                               T *y, int2 *meta, T *zstash, T *rectb, int tid) {
+  const int lane = tid & 31, w = tid >> 5, nw = blockDim.x >> 5;
   const int q = lane >> 3, j = lane & 7;
   int nlo, npr;
   stage_issue(st, 0, tid);
   stage_row_meta(lo_g, ptr_g, base, st.blk[0].x, st.blk[1].x, lane, nlo, npr);
   for (int b = 0; b < nblk; b++) {
     const int r0 = st.blk[b].x, nb = st.blk[b + 1].x - r0;
-    const int my_lo = nlo, my_pr = npr;
     if (w == 0) meta[lane] = make_int2(nlo, npr);
     if (b + 1 < nblk) {
       stage_issue(st, b + 1, tid);
@@ -818,7 +926,7 @@ __device__ bool staged_forward(Stage<T> &st, int nblk, const int32_t *lo_g, cons
     }
     const bool late = !stage_wait(st, b);
     if (__syncthreads_or(late)) return false;
-    const T *S = ((b & 1) ? st.buf1 : st.buf0) - stage_a0(st, b);  // S[e]: entry e of the envelope
+    const T *S = stage_block(st, b);
     for (int g = w; 4 * g < nb; g += nw) {
       const int t = 4 * g + q;
       const int2 mt = t < nb ? meta[t] : make_int2(r0, 0);
@@ -841,52 +949,103 @@ __device__ bool staged_forward(Stage<T> &st, int nblk, const int32_t *lo_g, cons
       if (j == 0 && t < nb) rectb[t] = acc;
     }
     __syncthreads();
-    if (kInv && w == 0) {
-      // y_b = (I + N) v with v = y_b - (the sums left of the block): lane t
-      // sums N_tj v_j over j in four chunks of 8 columns, one accumulator
-      // per chunk, in ascending j; no chain from row to row
-      const int2 ml = meta[nb - 1];
-      const T *N = S + ml.y + max(0, r0 - ml.x);  // after the block's left parts
-      const T *Nr = N + ((lane * (lane - 1)) >> 1);
-      T *vb = rectb + kSB;
-      const T v = lane < nb ? csub(y[r0 + lane], rectb[lane]) : czero<T>();
-      vb[lane] = v;
-      __syncwarp();
-      T acc[4] = {czero<T>(), czero<T>(), czero<T>(), czero<T>()};
+    if (w == 0) forward_triangle<T, kInv>(S, r0, nb, meta, y, zstash, rectb, lane);
+    __syncthreads();
+  }
+  return true;
+}
+
+// The same sums with the next block's rows taken ahead.  The triangle is one
+// warp's chain; while warp 0 walks it, the other warps take the next block's
+// rows up to its first column, and only that block's own columns are left for
+// after it: two barriers per block instead of three, and the row pass off the
+// chain.  It costs a second, short pass per row, so it pays where the chain
+// and not the issue slots bound the sweep.  Per phase, without and with: 59
+// subdomains of up to 600 elements, FP64 143 and 123 us; 123 of up to 1000,
+// FP32 326 and 254 us; 2253 of up to 1000, FP32 851 and 905 us.  Which it is
+// depends on the subdomains' sizes, their number and the precision, so the
+// first solve times both.
+template <typename T, bool kInv, int kNW>
+__device__ bool staged_forward_ahead(Stage<T> &st, int nblk, const int32_t *lo_g, const int64_t *ptr_g, int64_t base,
+                                     T *y, int2 *meta, T *zstash, T *rectb, int tid) {
+  const int lane = tid & 31, w = tid >> 5;
+  const int q = lane >> 3, j = lane & 7;
+  // row groups of four, shared by the warps after the first
+  constexpr int kStep = kNW - 1;
+  constexpr int kGroups = (kSB / 4 + kStep - 1) / kStep;
+  stage_issue(st, 0, tid);
+  if (nblk > 1) stage_issue(st, 1, tid);
+  if (w == 0) {
+    for (int b = 0; b < 2 && b < nblk; b++) {
+      int lo, pr;
+      stage_row_meta(lo_g, ptr_g, base, st.blk[b].x, st.blk[b + 1].x, lane, lo, pr);
+      meta[b * kSB + lane] = make_int2(lo, pr);
+    }
+    rectb[lane] = czero<T>();
+  }
+  __syncthreads();
+  for (int b = 0; b < nblk; b++) {
+    const int r0 = st.blk[b].x, nb = st.blk[b + 1].x - r0;
+    const bool next = b + 1 < nblk, next2 = b + 2 < nblk;
+    const int r1 = r0 + nb, nb1 = next ? st.blk[b + 2].x - r1 : 0;
+    int lo2 = 0, pr2 = 0;  // the row table of block b + 2
+    if (w == 0 && next2) stage_row_meta(lo_g, ptr_g, base, st.blk[b + 2].x, st.blk[b + 3].x, lane, lo2, pr2);
+    const int2 *m1 = meta + ((b + 1) & 1) * kSB;
+    T acc[kGroups];
+    bool late = false;
+    if (w == 0) {
+      late = !stage_wait(st, b);
+      forward_triangle<T, kInv>(stage_block(st, b), r0, nb, meta + (b & 1) * kSB, y, zstash, rectb, lane);
+    } else if (next) {
+      late = !stage_wait(st, b + 1);
+      const T *S1 = stage_block(st, b + 1);
 #pragma unroll
-      for (int jj = 0; jj < 8; jj++) {
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
-          const int j = 8 * c + jj;  // straight-line code: the loads go ahead of the sums
-          const T a = (j < lane && lane < nb) ? Nr[j] : czero<T>();
-          acc[c] = cmac(acc[c], a, vb[j]);
+      for (int u = 0; u < kGroups; u++) {
+        acc[u] = czero<T>();
+        const int t = 4 * (w - 1 + u * kStep) + q;
+        const int2 mt = t < nb1 ? m1[t] : make_int2(r0, 0);
+        const int len = t < nb1 ? max(0, r0 - mt.x) : 0;
+        int longest = max(len, __shfl_xor_sync(0xffffffffu, len, 8));
+        longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, 16));
+        const T *row = S1 + mt.y;
+        const T *yr = y + mt.x;
+        for (int k = j; k < longest; k += 16) {
+          const bool i0 = k < len, i1 = k + 8 < len;
+          const T a0 = i0 ? row[k] : czero<T>(), b0 = i0 ? yr[k] : czero<T>();
+          const T a1 = i1 ? row[k + 8] : czero<T>(), b1 = i1 ? yr[k + 8] : czero<T>();
+          acc[u] = cmac(acc[u], a0, b0);
+          acc[u] = cmac(acc[u], a1, b1);
         }
       }
-      const T val = cadd(v, cadd(cadd(acc[0], acc[1]), cadd(acc[2], acc[3])));
-      if (lane < nb) {
-        y[r0 + lane] = val;
-        zstash[r0 + lane] = cmul(val, N[((nb * (nb - 1)) >> 1) + lane]);  // the pivots' 1/d after N
-      }
-    } else if (w == 0) {
-      const T rect = rectb[lane];
-      T val = lane < nb ? csub(y[r0 + lane], rect) : czero<T>();
-      const T *mine = S + my_pr - my_lo;  // mine[col]: this lane's row at column col
-      for (int j0 = 0; j0 < nb - 1; j0 += 4) {
-        T op[4];
+    }
+    if (__syncthreads_or(late)) return false;
+    if (next2) {
+      stage_issue(st, b + 2, tid);
+      if (w == 0) meta[(b & 1) * kSB + lane] = make_int2(lo2, pr2);
+    }
+    if (next && w > 0) {
+      const T *S1 = stage_block(st, b + 1);
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
-          const int jj = j0 + u;
-          op[u] = (lane > jj && r0 + jj >= my_lo) ? mine[r0 + jj] : czero<T>();
-        }
+      for (int u = 0; u < kGroups; u++) {
+        const int t = 4 * (w - 1 + u * kStep) + q;
+        if (4 * (w - 1 + u * kStep) >= nb1) continue;
+        const int2 mt = t < nb1 ? m1[t] : make_int2(r1, 0);
+        const int done = max(0, r0 - mt.x), len = t < nb1 ? max(0, r1 - mt.x) : 0;
+        const T *row = S1 + mt.y;
+        const T *yr = y + mt.x;
+        // the lane's entries in the block's columns: at most kSB / 8 of them
+        int k = done + ((j - done) & 7);
+        T s = acc[u];
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
-          const T yj = shfl_idx(val, min(j0 + u, 31));
-          val = cmsub(val, op[u], yj);
+        for (int e = 0; e < kSB / 8; e++, k += 8) {
+          const bool in = k < len;
+          const T a0 = in ? row[k] : czero<T>(), b0 = in ? yr[k] : czero<T>();
+          s = cmac(s, a0, b0);
         }
-      }
-      if (lane < nb) {
-        y[r0 + lane] = val;
-        zstash[r0 + lane] = cmul(val, mine[r0 + lane]);  // 1/d on the diagonal
+        s = cadd(s, shfl_xor(s, 4));
+        s = cadd(s, shfl_xor(s, 2));
+        s = cadd(s, shfl_xor(s, 1));
+        if (j == 0 && t < nb1) rectb[t] = s;
       }
     }
     __syncthreads();
@@ -894,29 +1053,50 @@ __device__ bool staged_forward(Stage<T> &st, int nblk, const int32_t *lo_g, cons
   return true;
 }
 
+// The columns [cb, c1) of one 32-column chunk: the lane of column c applies
+// y_c -= L_tc x_t for a block's rows t from the last to the first, in place,
+// as the reference does (advlas_skyline.c:157-165); a group of eight rows
+// none of which reaches the chunk is skipped.
+template <typename T>
+__device__ __forceinline__ void backward_columns(const T *S, const int2 *m, const T *x, T *y, int nb, int cb, int c1,
+                                                 int lane) {
+  const int c = cb + lane;
+  const bool act = c < c1;
+  const uint32_t reach = __ballot_sync(0xffffffffu, lane < nb && m[lane].x < cb + 32);
+  T yc = act ? y[c] : czero<T>();
+  for (int t0 = (nb - 1) & ~7; t0 >= 0; t0 -= 8) {
+    if (((reach >> t0) & 0xffu) == 0) continue;
+    T v[8], xv[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+      const int t = t0 + 7 - u;
+      const int2 mt = m[t];
+      const int d = c - mt.x;
+      v[u] = (t < nb && act && d >= 0) ? S[mt.y + d] : czero<T>();
+      xv[u] = t < nb ? x[t] : czero<T>();  // x past the block may hold anything
+    }
+#pragma unroll
+    for (int u = 0; u < 8; u++) yc = cmsub(yc, v[u], xv[u]);
+  }
+  if (act) y[c] = yc;
+}
+
 // Backward sweep, blocks from the last.  Per block: the triangle with lanes
 // over the block's columns (warp 0), then the columns left of the block in
-// 32-column chunks shared out over the warps: the lane of column c applies
-// y_c -= L_tc x_t for the block's rows t from the last to the first, in
-// place, as the reference does (advlas_skyline.c:157-165); a group of eight
-// rows none of which reaches the chunk is skipped.
+// 32-column chunks shared out over the warps (backward_columns).  The stride
+// over the chunks is the block's size at run time: 2253 subdomains with FP32
+// factors took 917 us per phase with the warps a template argument, and 851
+// us so.
 template <typename T, bool kInv>
 __device__ bool staged_backward(Stage<T> &st, int nblk, const int32_t *lo_g, const int64_t *ptr_g, int64_t base,
-                                T *y, T *xb, int2 *meta, int *gmin, int tid, int nw) {
+                                T *y, T *xb, int2 *meta, int tid) {
   const int lane = tid & 31, w = tid >> 5;
   int nlo, npr;
   stage_row_meta(lo_g, ptr_g, base, st.blk[nblk - 1].x, st.blk[nblk].x, lane, nlo, npr);
   for (int b = nblk - 1; b >= 0; b--) {
     const int r0 = st.blk[b].x, nb = st.blk[b + 1].x - r0;
-    const int my_lo = nlo;
-    if (w == 0) {
-      meta[lane] = make_int2(nlo, npr);
-      int m = lane < nb ? nlo : INT_MAX;
-      m = min(m, __shfl_xor_sync(0xffffffffu, m, 1));
-      m = min(m, __shfl_xor_sync(0xffffffffu, m, 2));
-      m = min(m, __shfl_xor_sync(0xffffffffu, m, 4));
-      if ((lane & 7) == 0) gmin[lane >> 3] = m;
-    }
+    const int bmin = __reduce_min_sync(0xffffffffu, lane < nb ? nlo : INT_MAX);
+    if (w == 0) meta[lane] = make_int2(nlo, npr);
     // the forward sweep left blocks nblk-1 and nblk-2 in the buffers
     if (b >= 1) {
       if (b - 1 < nblk - 2) stage_issue(st, b - 1, tid);
@@ -924,89 +1104,73 @@ __device__ bool staged_backward(Stage<T> &st, int nblk, const int32_t *lo_g, con
     }
     const bool late = !stage_wait(st, b);
     if (__syncthreads_or(late)) return false;
-    const T *S = ((b & 1) ? st.buf1 : st.buf0) - stage_a0(st, b);
-    if (kInv && w == 0) {
-      // x_b = (I + N)^T w with w = y_b: lane j sums N_tj w_t over t in four
-      // chunks of 8 rows, one accumulator per chunk, in ascending t
-      const int2 ml = meta[nb - 1];
-      const T *N = S + ml.y + max(0, r0 - ml.x);
-      const T wv = lane < nb ? y[r0 + lane] : czero<T>();
-      T acc[4] = {czero<T>(), czero<T>(), czero<T>(), czero<T>()};
-#pragma unroll
-      for (int tt = 0; tt < 8; tt++) {
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
-          const int t = 8 * c + tt;
-          const T a = (lane < t && t < nb) ? N[((t * (t - 1)) >> 1) + lane] : czero<T>();
-          acc[c] = cmac(acc[c], a, y[r0 + min(t, nb - 1)]);
-        }
-      }
-      const T val = cadd(wv, cadd(cadd(acc[0], acc[1]), cadd(acc[2], acc[3])));
-      __syncwarp();  // every lane has read y_b before it is overwritten
-      if (lane < nb) {
-        y[r0 + lane] = val;
-        xb[lane] = val;
-      }
-    } else if (w == 0) {
-      // triangle, lanes over the block's columns; operands of 4 steps loaded ahead
-      T val = lane < nb ? y[r0 + lane] : czero<T>();
-      const int col = r0 + lane;
-      for (int i0 = nb - 1; i0 >= 1; i0 -= 4) {
-        T op[4];
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-          const int i = i0 - u;
-          const int2 mt = meta[max(i, 0)];
-          op[u] = (i >= 1 && lane < i && col >= mt.x) ? S[mt.y + col - mt.x] : czero<T>();
-        }
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-          const T xi = shfl_idx(val, max(i0 - u, 0));
-          val = cmsub(val, op[u], xi);
-        }
-      }
-      if (lane < nb) {
-        y[r0 + lane] = val;
-        xb[lane] = val;
-      }
-    }
-    int bmin = lane < nb ? my_lo : INT_MAX;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) bmin = min(bmin, __shfl_xor_sync(0xffffffffu, bmin, o));
+    const T *S = stage_block(st, b);
+    if (w == 0) backward_triangle<T, kInv>(S, r0, nb, meta, y, xb, lane);
     __syncthreads();
-    for (int cb = bmin + 32 * w; cb < r0; cb += 32 * nw) {
-      const int c = cb + lane;
-      const bool act = c < r0;
-      T yc = act ? y[c] : czero<T>();
-      for (int t0 = (nb - 1) & ~7; t0 >= 0; t0 -= 8) {
-        if (gmin[t0 >> 3] >= cb + 32) continue;  // no row of the group reaches this chunk
-        T v[8], xv[8];
-#pragma unroll
-        for (int u = 0; u < 8; u++) {
-          const int t = t0 + 7 - u;
-          const int2 mt = meta[t];
-          const int d = c - mt.x;
-          v[u] = (t < nb && act && d >= 0) ? S[mt.y + d] : czero<T>();
-          xv[u] = t < nb ? xb[t] : czero<T>();  // xb past the block may hold anything
-        }
-#pragma unroll
-        for (int u = 0; u < 8; u++) yc = cmsub(yc, v[u], xv[u]);
-      }
-      if (act) y[c] = yc;
-    }
+    for (int cb = bmin + 32 * w; cb < r0; cb += blockDim.x) backward_columns(S, meta, xb, y, nb, cb, r0, lane);
     __syncthreads();
   }
   return true;
 }
 
-template <typename T, bool kInv>
-__global__ void __launch_bounds__(128) subsolve_staged_kernel(DevProblem p, int mode, const double2 *rhs, double2 *xout,
-                                                             T *zstash, int accumulate, StageLayout lay) {
+// The same with the chain taken ahead: warp 0 takes the columns of the block
+// before and then that block's triangle, while the other warps take the rest
+// of the columns: one barrier per block.
+template <typename T, bool kInv, int kNW>
+__device__ bool staged_backward_ahead(Stage<T> &st, int nblk, const int32_t *lo_g, const int64_t *ptr_g, int64_t base,
+                                      T *y, T *xb, int2 *meta, int tid) {
+  const int lane = tid & 31, w = tid >> 5;
+  // the forward sweep left blocks nblk-1 and nblk-2, and their row tables
+  bool late = false;
+  if (w == 0) {
+    const int b = nblk - 1, r0 = st.blk[b].x;
+    late = !stage_wait(st, b);
+    backward_triangle<T, kInv>(stage_block(st, b), r0, st.blk[b + 1].x - r0, meta + (b & 1) * kSB, y,
+                               xb + (b & 1) * kSB, lane);
+  }
+  if (__syncthreads_or(late)) return false;
+  for (int b = nblk - 1; b >= 1; b--) {
+    const int r0 = st.blk[b].x, nb = st.blk[b + 1].x - r0, rp = st.blk[b - 1].x;
+    const int2 *m = meta + (b & 1) * kSB;
+    const T *S = stage_block(st, b), *x = xb + (b & 1) * kSB;
+    late = false;
+    int lo2 = 0, pr2 = 0;  // the row table of block b - 2
+    if (w == 0) {
+      if (b >= 2) stage_row_meta(lo_g, ptr_g, base, st.blk[b - 2].x, st.blk[b - 1].x, lane, lo2, pr2);
+      backward_columns(S, m, x, y, nb, rp, r0, lane);
+      __syncwarp();
+      late = !stage_wait(st, b - 1);
+      backward_triangle<T, kInv>(stage_block(st, b - 1), rp, r0 - rp, meta + ((b - 1) & 1) * kSB, y,
+                                 xb + ((b - 1) & 1) * kSB, lane);
+    } else {
+      const int bmin = __reduce_min_sync(0xffffffffu, lane < nb ? m[lane].x : INT_MAX);
+      for (int cb = bmin + 32 * (w - 1); cb < rp; cb += 32 * (kNW - 1)) backward_columns(S, m, x, y, nb, cb, rp, lane);
+    }
+    if (__syncthreads_or(late)) return false;
+    if (b >= 2) {
+      stage_issue(st, b - 2, tid);
+      if (w == 0) {
+        meta[(b & 1) * kSB + lane] = make_int2(lo2, pr2);
+        __syncwarp();
+      }
+    }
+  }
+  return true;
+}
+
+// kAhead: 0 for the plain sweeps with one, two or four warps, otherwise the
+// number of warps of the sweeps that take the rows ahead.
+template <typename T, bool kInv, int kAhead>
+__global__ void __launch_bounds__(kAhead ? 32 * kAhead : 128)
+    subsolve_staged_kernel(DevProblem p, int mode, const double2 *rhs, double2 *xout, T *zstash, int accumulate,
+                           StageLayout lay) {
   if (mode == kModeIter && p.sc->status != 0) return;
   if (accumulate && refine_skipped(p, mode)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ double red[4][2];
-  const int tid = threadIdx.x, nt = blockDim.x, nw = nt >> 5;
+  constexpr int kMaxWarps = kAhead ? kAhead : 4;
+  __shared__ double red[kMaxWarps][2];
+  const int nt = kAhead ? 32 * kAhead : blockDim.x, nw = nt >> 5;
+  const int tid = threadIdx.x;
   const int s = p.sub_order[blockIdx.x];
   const int64_t io = p.int_off[s];
   const int nI = (int)(p.int_off[s + 1] - io);
@@ -1015,10 +1179,8 @@ __global__ void __launch_bounds__(128) subsolve_staged_kernel(DevProblem p, int 
   const int nblk = blk_off[s + 1] - b0 - 1;
   if (nI == 0 || nblk <= 0) return;
   T *y = (T *)(smem_raw + lay.y);
-  T *xb = (T *)(smem_raw + lay.xb);
   T *rectb = (T *)(smem_raw + lay.rb);
   int2 *meta = (int2 *)(smem_raw + lay.meta);
-  int *gmin = (int *)(smem_raw + lay.gmin);
   int2 *blk = (int2 *)(smem_raw + lay.blk);
   Stage<T> st;
   st.buf0 = (T *)(smem_raw + lay.buf0);
@@ -1042,6 +1204,7 @@ __global__ void __launch_bounds__(128) subsolve_staged_kernel(DevProblem p, int 
   }
   // right-hand side; a refinement step is skipped when its residual is already small
   double rn = 0.0, bn = 0.0;
+#pragma unroll 4
   for (int c = tid; c < nI; c += nt) {
     const double2 r = rhs[io + c];
     y[c] = from_d2<T>(r);
@@ -1063,7 +1226,9 @@ __global__ void __launch_bounds__(128) subsolve_staged_kernel(DevProblem p, int 
       red[tid >> 5][1] = bn;
     }
     __syncthreads();
-    for (int k = 0; k < nw; k++) {
+#pragma unroll
+    for (int k = 0; k < kMaxWarps; k++) {
+      if (k >= nw) break;
       rn = fmax(rn, red[k][0]);
       bn = fmax(bn, red[k][1]);
     }
@@ -1076,16 +1241,25 @@ __global__ void __launch_bounds__(128) subsolve_staged_kernel(DevProblem p, int 
   // backward sweep's reads are the last use
   st.hint = 1;
   st.policy = l2_evict_last();
-  bool ok = staged_forward<T, kInv>(st, nblk, lo_g, ptr_g, base, y, meta, z, rectb, tid, nw);
+  bool ok;
+  if constexpr (kAhead != 0)
+    ok = staged_forward_ahead<T, kInv, kAhead>(st, nblk, lo_g, ptr_g, base, y, meta, z, rectb, tid);
+  else
+    ok = staged_forward<T, kInv>(st, nblk, lo_g, ptr_g, base, y, meta, z, rectb, tid);
   if (ok) {
+#pragma unroll 4
     for (int c = tid; c < nI; c += nt) y[c] = z[c];
     __syncthreads();
     st.policy = l2_evict_first();
-    ok = staged_backward<T, kInv>(st, nblk, lo_g, ptr_g, base, y, xb, meta, gmin, tid, nw);
+    if constexpr (kAhead != 0)
+      ok = staged_backward_ahead<T, kInv, kAhead>(st, nblk, lo_g, ptr_g, base, y, rectb, meta, tid);
+    else
+      ok = staged_backward<T, kInv>(st, nblk, lo_g, ptr_g, base, y, rectb, meta, tid);
   }
   // every copy issued into this CTA's shared memory has landed before it exits
   stage_drain(st);
   if (!ok) return;
+#pragma unroll 4
   for (int c = tid; c < nI; c += nt) {
     double2 x = make_double2((double)y[c].x, (double)y[c].y);
     if (accumulate) x = cadd(xout[io + c], x);
@@ -1737,6 +1911,15 @@ size_t subsolve_smem_bytes(int max_interior, int max_iface, bool fp32) {
   return cta_smem_bytes(max_interior, max_iface, fp32);
 }
 
+template <typename T, bool kInv>
+void launch_staged_sweep(const DevProblem &p, int mode, const double2 *rhs, double2 *xout, T *zstash, int accumulate,
+                         const StageLayout &lay, cudaStream_t stream) {
+  const auto kernel = !p.stage_ahead         ? subsolve_staged_kernel<T, kInv, 0>
+                      : p.stage_warps == 8 ? subsolve_staged_kernel<T, kInv, 8>
+                                           : subsolve_staged_kernel<T, kInv, 4>;
+  kernel<<<p.nsub, 32 * p.stage_warps, lay.total, stream>>>(p, mode, rhs, xout, zstash, accumulate, lay);
+}
+
 template <bool kInv>
 void launch_staged(const DevProblem &p, int mode, bool fp32, cudaStream_t stream) {
   const StageLayout lay = kInv ? stage_layout(p.max_interior, p.inv_max_blocks, p.inv_cap, fp32)
@@ -1747,13 +1930,13 @@ void launch_staged(const DevProblem &p, int mode, bool fp32, cudaStream_t stream
   // thread beat lanes sharing a row (timed with 1, 2, 4 and 8 lanes)
   launch_chained(rhs_kernel<1>, blocks_min1(p.n_interior, 256), 256, 0, stream, p, mode, rhs);
   if (fp32) {
-    subsolve_staged_kernel<float2, kInv><<<p.nsub, 32 * p.stage_warps, lay.total, stream>>>(p, mode, p.B, p.Y, p.Y32, 0, lay);
+    launch_staged_sweep<float2, kInv>(p, mode, p.B, p.Y, p.Y32, 0, lay, stream);
     for (int k = 0; k < p.ir_steps; k++) {
       ir_residual_kernel<4><<<blocks_min1(p.n_interior * 4, 256), 256, 0, stream>>>(p, mode);
-      subsolve_staged_kernel<float2, kInv><<<p.nsub, 32 * p.stage_warps, lay.total, stream>>>(p, mode, p.Rres, p.Y, p.Y32, 1, lay);
+      launch_staged_sweep<float2, kInv>(p, mode, p.Rres, p.Y, p.Y32, 1, lay, stream);
     }
   } else {
-    subsolve_staged_kernel<double2, kInv><<<p.nsub, 32 * p.stage_warps, lay.total, stream>>>(p, mode, p.Y, p.Y, p.Y, 0, lay);
+    launch_staged_sweep<double2, kInv>(p, mode, p.Y, p.Y, p.Y, 0, lay, stream);
   }
   iface_product_kernel<1><<<blocks_min1(p.n_slots, 256), 256, 0, stream>>>(p, mode);
 }
@@ -1811,14 +1994,24 @@ int raise_smem_limit(const void *func, int slot, size_t smem) {
   return 0;
 }
 
+namespace {
+template <typename T, bool kInv>
+int configure_sweep(int slot, size_t smem) {
+  const void *const f[kSweepVariants] = {(const void *)subsolve_staged_kernel<T, kInv, 0>,
+                                         (const void *)subsolve_staged_kernel<T, kInv, 4>,
+                                         (const void *)subsolve_staged_kernel<T, kInv, 8>};
+  for (int k = 0; k < kSweepVariants; k++)
+    if (const int rc = raise_smem_limit(f[k], slot + k, smem)) return rc;
+  return 0;
+}
+}  // namespace
+
 int configure_subsolve_staged(size_t smem, bool fp32) {
-  return fp32 ? raise_smem_limit((const void *)subsolve_staged_kernel<float2, false>, kSlotStaged32, smem)
-              : raise_smem_limit((const void *)subsolve_staged_kernel<double2, false>, kSlotStaged64, smem);
+  return fp32 ? configure_sweep<float2, false>(kSlotStaged32, smem) : configure_sweep<double2, false>(kSlotStaged64, smem);
 }
 
 int configure_subsolve_inv(size_t smem, bool fp32) {
-  return fp32 ? raise_smem_limit((const void *)subsolve_staged_kernel<float2, true>, kSlotInv32, smem)
-              : raise_smem_limit((const void *)subsolve_staged_kernel<double2, true>, kSlotInv64, smem);
+  return fp32 ? configure_sweep<float2, true>(kSlotInv32, smem) : configure_sweep<double2, true>(kSlotInv64, smem);
 }
 
 void launch_inv_relayout(const DevProblem &p, const double2 *L64, bool fp32, cudaStream_t stream) {

@@ -90,7 +90,8 @@ struct DevProblem {
   const int2 *blk_tab;           // per subdomain nblk+1 x (first row, first envelope element)
   int32_t max_blocks;            // most blocks of one subdomain
   int32_t stage_cap;             // envelope elements per staging buffer
-  int32_t stage_warps;           // warps sharing one subdomain's sweeps (1, 2 or 4)
+  int32_t stage_warps;           // warps sharing one subdomain's sweeps (1, 2, 4, or 8 with stage_ahead)
+  int32_t stage_ahead;           // the sweeps take the next block's rows ahead of the triangle's end (4 or 8 warps)
   // staged solve on the block-inverse layout (kSolveInv): per block of rows,
   // the rows' entries left of the block, then N = (I + L_bb)^-1 - I strictly
   // lower and row-major (row t at t(t-1)/2), then the block's pivots 1/d
@@ -211,17 +212,18 @@ void launch_inv_relayout(const DevProblem &p, const double2 *L64, bool fp32, cud
 // the current device; `slot` names the kernel.
 // Slots of the process-wide dynamic shared-memory limits (raise_smem_limit):
 // one per kernel instantiation that runs above the 48 KB default.
+constexpr int kSweepVariants = 3;  // the plain staged sweep; with the rows taken ahead by 4 and by 8 warps
 enum SmemSlot {
   kSlotStaged32 = 0,
-  kSlotStaged64 = 1,
-  kSlotCta32 = 2,
-  kSlotCta64 = 3,
-  kSlotInv32 = 4,
-  kSlotInv64 = 5,
-  kSlotMulti32 = 6,
-  kSlotMulti64 = 7,
-  kSlotFactor = 8,
-  kSmemSlots = 9
+  kSlotStaged64 = kSlotStaged32 + kSweepVariants,
+  kSlotInv32 = kSlotStaged64 + kSweepVariants,
+  kSlotInv64 = kSlotInv32 + kSweepVariants,
+  kSlotCta32 = kSlotInv64 + kSweepVariants,
+  kSlotCta64,
+  kSlotMulti32,
+  kSlotMulti64,
+  kSlotFactor,
+  kSmemSlots
 };
 int raise_smem_limit(const void *func, int slot, size_t smem);
 // kernels one launch_subsolve call issues

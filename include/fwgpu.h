@@ -156,7 +156,7 @@ typedef struct {
 
 /* Batched subdomain-solve kernels.  AUTO runs the WARP kernel (FP64
  * factors) or the BLOCKINV kernel (FP32 factors) at the staging capacity
- * that a rule on the envelope gives, and times 1, 2 and 4 warps per
+ * that a rule on the envelope gives, and times 2, 4 and 8 warps per
  * subdomain, which sum in the same order; WARP also times its staging
  * capacities, which changes the order of the sums. */
 #define FWGPU_SOLVE_AUTO 0

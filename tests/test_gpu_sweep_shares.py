@@ -1,0 +1,24 @@
+"""The staged sweeps with one, two and four warps per subdomain and with the
+timed choice (which may take the rows ahead, with four or eight warps) give
+the same bits: subdomains of one row block, of a few, and of one of many."""
+import numpy as np
+import pytest
+
+from adventure_fullwave_b200 import hddm, meshgen
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,leaf", [(4, 7), (5, 30), (6, 110), (8, 600), (8, 3072)])
+@pytest.mark.parametrize("precision,kernel", [("fp64", "auto"), ("fp64", "blockinv"), ("fp32_ir", "auto")])
+def test_same_bits_for_every_share(n, leaf, precision, kernel):
+    model = meshgen.make_model("w", n=n, size=1.0, npml=1, layers=2, nleaves=None, leaf_cap=leaf, jitter=(0.3, 0.7),
+                               seed=5)
+    meshgen.round_trip_material(model)
+    got = []
+    for warps in (1, 2, 4, 0):
+        x, r = hddm.hddm_solver_CS(model, 0, hddm_eps=1e-9, hddm_max_loop=40, precision=precision, solve_kernel=kernel,
+                                   stage_warps=warps)
+        got.append((np.asarray(x), r.iterations))
+    for x, its in got[1:]:
+        assert its == got[0][1] and np.array_equal(x, got[0][0], equal_nan=True)
