@@ -119,6 +119,7 @@ struct fwgpu_context {
   int2 *d_blk_tab = nullptr;
   // block-inverse layout of the factor (FWGPU_SOLVE_BLOCKINV)
   bool inv_ok = false;             // its block table is built and its kernel fits in shared memory
+  bool inv_ahead_ok = false;       // with room for the sweeps that take rows ahead
   int64_t inv_len = 0;             // elements of Linv
   int64_t *d_inv_ptr = nullptr;
   int32_t *d_inv_blk_off = nullptr;
@@ -126,6 +127,7 @@ struct fwgpu_context {
   double2 *d_Linv64 = nullptr;
   float2 *d_Linv32 = nullptr;
   std::vector<int> stage_caps;     // staging capacities that fit in shared memory
+  std::vector<int> stage_ahead_caps;  // those with room for the sweeps that take rows ahead
   std::vector<int32_t> h_order;    // subdomains by interior size, largest first (the device sub_order)
   std::vector<int32_t> h_nblk;     // staged blocks of each subdomain at the current capacity
   int64_t launches = 0;            // kernels launched since the last reset
@@ -1012,6 +1014,18 @@ static int build_stage_blocks(fwgpu_context *c, int cap, int *max_blocks_out) {
   return FWGPU_OK;
 }
 
+// The staged sweeps' row table for one layout's row positions, kept with the
+// layout.
+static int build_row_table(fwgpu_context *c, const int64_t *d_ptr, const int2 **out) {
+  int2 *tab = nullptr;
+  FW_TRY(c->alloc(&tab, c->p.sub_int_off[c->m.nsub]));
+  fw::launch_row_table(c->dp, d_ptr, tab, c->stream);
+  FW_CUDA(cudaGetLastError());
+  c->launches += 1;
+  *out = tab;
+  return FWGPU_OK;
+}
+
 // Block-inverse layout: row blocks of at most 32 rows whose stored elements
 // (the rows' entries left of the block, the block's N = (I + L_bb)^-1 - I as
 // a dense strict lower triangle, and its pivots) fit one staging buffer of
@@ -1061,7 +1075,7 @@ static int build_inv_blocks(fwgpu_context *c, int cap) {
     max_blocks = std::max(max_blocks, nb);
   }
   boff[nsub] = (int32_t)btab.size();
-  const size_t smem = fw::subsolve_staged_smem_bytes(max_nI, max_blocks, cap, fp32);
+  const size_t smem = fw::subsolve_staged_smem_bytes(max_nI, max_blocks, cap, fp32, false);
   if (smem > 227 * 1024 || fw::configure_subsolve_inv(smem, fp32) != 0) {
     c->inv_ok = false;
     return FWGPU_OK;
@@ -1076,12 +1090,14 @@ static int build_inv_blocks(fwgpu_context *c, int cap) {
     FW_TRY(c->alloc(&c->d_Linv64, pos + 64));
   c->inv_len = pos;
   c->dp.inv_ptr = c->d_inv_ptr;
+  FW_TRY(build_row_table(c, c->d_inv_ptr, &c->dp.inv_row_tab));
   c->dp.inv_blk_off = c->d_inv_blk_off;
   c->dp.inv_blk_tab = c->d_inv_blk_tab;
   c->dp.Linv64 = c->d_Linv64;
   c->dp.Linv32 = c->d_Linv32;
   c->dp.inv_max_blocks = max_blocks;
   c->dp.inv_cap = cap;
+  c->inv_ahead_ok = fw::subsolve_staged_smem_bytes(max_nI, max_blocks, cap, fp32, true) <= 227 * 1024;
   c->inv_ok = true;
   return FWGPU_OK;
 }
@@ -1096,15 +1112,18 @@ static int setup_stage(fwgpu_context *c) {
   std::vector<int> cand = fp32 ? std::vector<int>{1024, 1536, 2048, 3072} : std::vector<int>{512, 768, 1024, 1536};
   if (c->opts.stage_cap > 0) cand = {c->opts.stage_cap};
   c->stage_caps.clear();
+  c->stage_ahead_caps.clear();
   size_t smem_max = 0;
   for (int cap : cand) {
     cap = std::max(cap, min_cap);
     if (std::find(c->stage_caps.begin(), c->stage_caps.end(), cap) != c->stage_caps.end()) continue;
     int mb = 0;
     FW_TRY(build_stage_blocks(c, cap, &mb));
-    const size_t smem = fw::subsolve_staged_smem_bytes(p.max_interior, mb, cap, fp32);
+    const size_t smem = fw::subsolve_staged_smem_bytes(p.max_interior, mb, cap, fp32, false);
     if (smem > 227 * 1024) continue;
     c->stage_caps.push_back(cap);
+    if (fw::subsolve_staged_smem_bytes(p.max_interior, mb, cap, fp32, true) <= 227 * 1024)
+      c->stage_ahead_caps.push_back(cap);
     smem_max = std::max(smem_max, smem);
   }
   c->warp_ok = !c->stage_caps.empty() && fw::configure_subsolve_staged(smem_max, fp32) == 0;
@@ -1140,8 +1159,11 @@ static int tune_solve_kernel(fwgpu_context *c) {
   // every way of sharing out a sweep that the caller's stage_warps allows;
   // AUTO leaves out one warp, which was never the fastest
   auto sweeps = [&](int variant, int cap) {
+    const bool room = variant == fw::kSolveInv ? c->inv_ahead_ok
+                                               : std::find(c->stage_ahead_caps.begin(), c->stage_ahead_caps.end(),
+                                                           cap) != c->stage_ahead_caps.end();
     for (int warps = 1; warps <= 8; warps *= 2)
-      for (int ahead = warps == 8 ? 1 : 0; ahead <= (warps >= 4 ? 1 : 0); ahead++)
+      for (int ahead = warps == 8 ? 1 : 0; ahead <= (warps >= 4 && room ? 1 : 0); ahead++)
         if (c->opts.stage_warps == warps || (c->opts.stage_warps == 0 && !(any && warps == 1)))
           cand.push_back({variant, cap, warps, ahead});
   };
@@ -1217,6 +1239,7 @@ int fwgpu_solve_dom_1st(fwgpu_context *c) {
     FW_TRY(c->alloc(&c->d_L64, pos + 64));
     c->dp.env_lo = c->d_env_lo;
     c->dp.env_ptr = c->d_env_ptr;
+    FW_TRY(build_row_table(c, c->d_env_ptr, &c->dp.row_tab));
     if (c->opts.precision == FWGPU_PREC_FP32_IR) FW_TRY(c->alloc(&c->d_L32, pos + 64));
     FW_TRY(setup_stage(c));
     if (c->opts.solve_kernel == FWGPU_SOLVE_WARP && !c->warp_ok)

@@ -761,7 +761,8 @@ struct StageLayout {
 };
 
 // Shared-memory slice of one subdomain warp of the staged solve.
-__host__ __device__ inline StageLayout stage_layout(int max_interior, int max_blocks, int cap, bool fp32) {
+__host__ __device__ inline StageLayout stage_layout(int max_interior, int max_blocks, int cap, bool fp32,
+                                                   bool ahead) {
   const size_t es = fp32 ? 8 : 16;
   StageLayout l;
   size_t o = 0;
@@ -774,7 +775,7 @@ __host__ __device__ inline StageLayout stage_layout(int max_interior, int max_bl
   l.rb = o;
   o += a16(2 * kSB * es);  // forward: row sums and a block's vector; backward: two blocks' solutions
   l.meta = o;
-  o += 2 * kSB * 8;        // two blocks' row tables
+  o += (ahead ? 4 : 2) * kSB * 8;  // row tables
   l.bar = o;
   o += 32;
   l.blk = o;
@@ -892,6 +893,11 @@ __device__ __forceinline__ void backward_triangle(const T *S, int r0, int nb, co
   }
 }
 
+// block b's row table: two for the plain sweeps (a block's and the next
+// one's), four for the sweeps that take rows ahead (three in use)
+__device__ __forceinline__ int2 *table2(int2 *meta, int b) { return meta + (b & 1) * kSB; }
+__device__ __forceinline__ int2 *table4(int2 *meta, int b) { return meta + (b & 3) * kSB; }
+
 // the staged block b, by envelope element
 template <typename T>
 __device__ __forceinline__ const T *stage_block(const Stage<T> &st, int b) {
@@ -910,26 +916,25 @@ __device__ __forceinline__ const T *stage_block(const Stage<T> &st, int b) {
 // Returns false when a staged copy did not arrive (error word raised); the
 // caller drains the copies in flight and stops.
 template <typename T, bool kInv>
-__device__ bool staged_forward(Stage<T> &st, int nblk, const int32_t *lo_g, const int64_t *ptr_g, int64_t base,
-                               T *y, int2 *meta, T *zstash, T *rectb, int tid) {
+__device__ bool staged_forward(Stage<T> &st, int nblk, const int2 *rows_g, T *y, int2 *meta, T *zstash, T *rectb,
+                               int tid) {
   const int lane = tid & 31, w = tid >> 5, nw = blockDim.x >> 5;
   const int q = lane >> 3, j = lane & 7;
-  int nlo, npr;
   stage_issue(st, 0, tid);
-  stage_row_meta(lo_g, ptr_g, base, st.blk[0].x, st.blk[1].x, lane, nlo, npr);
+  if (w == 0) rows_issue(st, rows_g, table2(meta, 0), 0, lane);
   for (int b = 0; b < nblk; b++) {
     const int r0 = st.blk[b].x, nb = st.blk[b + 1].x - r0;
-    if (w == 0) meta[lane] = make_int2(nlo, npr);
-    if (b + 1 < nblk) {
-      stage_issue(st, b + 1, tid);
-      stage_row_meta(lo_g, ptr_g, base, st.blk[b + 1].x, st.blk[b + 2].x, lane, nlo, npr);
-    }
+    const bool next = b + 1 < nblk;
+    const int2 *m = table2(meta, b);
+    if (next) stage_issue(st, b + 1, tid);
+    if (w == 0) rows_wait();
     const bool late = !stage_wait(st, b);
     if (__syncthreads_or(late)) return false;
+    if (w == 0 && next) rows_issue(st, rows_g, table2(meta, b + 1), b + 1, lane);
     const T *S = stage_block(st, b);
     for (int g = w; 4 * g < nb; g += nw) {
       const int t = 4 * g + q;
-      const int2 mt = t < nb ? meta[t] : make_int2(r0, 0);
+      const int2 mt = t < nb ? m[t] : make_int2(r0, 0);
       const int len = t < nb ? max(0, r0 - mt.x) : 0;
       int longest = max(len, __shfl_xor_sync(0xffffffffu, len, 8));
       longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, 16));
@@ -949,7 +954,7 @@ __device__ bool staged_forward(Stage<T> &st, int nblk, const int32_t *lo_g, cons
       if (j == 0 && t < nb) rectb[t] = acc;
     }
     __syncthreads();
-    if (w == 0) forward_triangle<T, kInv>(S, r0, nb, meta, y, zstash, rectb, lane);
+    if (w == 0) forward_triangle<T, kInv>(S, r0, nb, m, y, zstash, rectb, lane);
     __syncthreads();
   }
   return true;
@@ -966,8 +971,8 @@ __device__ bool staged_forward(Stage<T> &st, int nblk, const int32_t *lo_g, cons
 // depends on the subdomains' sizes, their number and the precision, so the
 // first solve times both.
 template <typename T, bool kInv, int kNW>
-__device__ bool staged_forward_ahead(Stage<T> &st, int nblk, const int32_t *lo_g, const int64_t *ptr_g, int64_t base,
-                                     T *y, int2 *meta, T *zstash, T *rectb, int tid) {
+__device__ bool staged_forward_ahead(Stage<T> &st, int nblk, const int2 *rows_g, T *y, int2 *meta, T *zstash,
+                                     T *rectb, int tid) {
   const int lane = tid & 31, w = tid >> 5;
   const int q = lane >> 3, j = lane & 7;
   // row groups of four, shared by the warps after the first
@@ -976,11 +981,8 @@ __device__ bool staged_forward_ahead(Stage<T> &st, int nblk, const int32_t *lo_g
   stage_issue(st, 0, tid);
   if (nblk > 1) stage_issue(st, 1, tid);
   if (w == 0) {
-    for (int b = 0; b < 2 && b < nblk; b++) {
-      int lo, pr;
-      stage_row_meta(lo_g, ptr_g, base, st.blk[b].x, st.blk[b + 1].x, lane, lo, pr);
-      meta[b * kSB + lane] = make_int2(lo, pr);
-    }
+    for (int b = 0; b < 2 && b < nblk; b++) rows_issue(st, rows_g, table4(meta, b), b, lane);
+    rows_wait();
     rectb[lane] = czero<T>();
   }
   __syncthreads();
@@ -988,14 +990,13 @@ __device__ bool staged_forward_ahead(Stage<T> &st, int nblk, const int32_t *lo_g
     const int r0 = st.blk[b].x, nb = st.blk[b + 1].x - r0;
     const bool next = b + 1 < nblk, next2 = b + 2 < nblk;
     const int r1 = r0 + nb, nb1 = next ? st.blk[b + 2].x - r1 : 0;
-    int lo2 = 0, pr2 = 0;  // the row table of block b + 2
-    if (w == 0 && next2) stage_row_meta(lo_g, ptr_g, base, st.blk[b + 2].x, st.blk[b + 3].x, lane, lo2, pr2);
-    const int2 *m1 = meta + ((b + 1) & 1) * kSB;
+    if (w == 0 && next2) rows_issue(st, rows_g, table4(meta, b + 2), b + 2, lane);
+    const int2 *m1 = table4(meta, b + 1);
     T acc[kGroups];
     bool late = false;
     if (w == 0) {
       late = !stage_wait(st, b);
-      forward_triangle<T, kInv>(stage_block(st, b), r0, nb, meta + (b & 1) * kSB, y, zstash, rectb, lane);
+      forward_triangle<T, kInv>(stage_block(st, b), r0, nb, table4(meta, b), y, zstash, rectb, lane);
     } else if (next) {
       late = !stage_wait(st, b + 1);
       const T *S1 = stage_block(st, b + 1);
@@ -1019,10 +1020,8 @@ __device__ bool staged_forward_ahead(Stage<T> &st, int nblk, const int32_t *lo_g
       }
     }
     if (__syncthreads_or(late)) return false;
-    if (next2) {
-      stage_issue(st, b + 2, tid);
-      if (w == 0) meta[(b & 1) * kSB + lane] = make_int2(lo2, pr2);
-    }
+    if (next2) stage_issue(st, b + 2, tid);
+    if (w == 0) rows_wait();
     if (next && w > 0) {
       const T *S1 = stage_block(st, b + 1);
 #pragma unroll
@@ -1088,26 +1087,23 @@ __device__ __forceinline__ void backward_columns(const T *S, const int2 *m, cons
 // factors took 917 us per phase with the warps a template argument, and 851
 // us so.
 template <typename T, bool kInv>
-__device__ bool staged_backward(Stage<T> &st, int nblk, const int32_t *lo_g, const int64_t *ptr_g, int64_t base,
-                                T *y, T *xb, int2 *meta, int tid) {
+__device__ bool staged_backward(Stage<T> &st, int nblk, const int2 *rows_g, T *y, T *xb, int2 *meta, int tid) {
   const int lane = tid & 31, w = tid >> 5;
-  int nlo, npr;
-  stage_row_meta(lo_g, ptr_g, base, st.blk[nblk - 1].x, st.blk[nblk].x, lane, nlo, npr);
   for (int b = nblk - 1; b >= 0; b--) {
     const int r0 = st.blk[b].x, nb = st.blk[b + 1].x - r0;
-    const int bmin = __reduce_min_sync(0xffffffffu, lane < nb ? nlo : INT_MAX);
-    if (w == 0) meta[lane] = make_int2(nlo, npr);
-    // the forward sweep left blocks nblk-1 and nblk-2 in the buffers
-    if (b >= 1) {
-      if (b - 1 < nblk - 2) stage_issue(st, b - 1, tid);
-      stage_row_meta(lo_g, ptr_g, base, st.blk[b - 1].x, st.blk[b].x, lane, nlo, npr);
-    }
+    const int2 *m = table2(meta, b);
+    // the forward sweep left blocks nblk-1 and nblk-2 in the buffers, and their row tables
+    const bool next = b >= 1 && b - 1 < nblk - 2;
+    if (next) stage_issue(st, b - 1, tid);
+    if (w == 0) rows_wait();
     const bool late = !stage_wait(st, b);
     if (__syncthreads_or(late)) return false;
+    if (w == 0 && next) rows_issue(st, rows_g, table2(meta, b - 1), b - 1, lane);
     const T *S = stage_block(st, b);
-    if (w == 0) backward_triangle<T, kInv>(S, r0, nb, meta, y, xb, lane);
+    if (w == 0) backward_triangle<T, kInv>(S, r0, nb, m, y, xb, lane);
+    const int bmin = __reduce_min_sync(0xffffffffu, lane < nb ? m[lane].x : INT_MAX);
     __syncthreads();
-    for (int cb = bmin + 32 * w; cb < r0; cb += blockDim.x) backward_columns(S, meta, xb, y, nb, cb, r0, lane);
+    for (int cb = bmin + 32 * w; cb < r0; cb += blockDim.x) backward_columns(S, m, xb, y, nb, cb, r0, lane);
     __syncthreads();
   }
   return true;
@@ -1117,43 +1113,36 @@ __device__ bool staged_backward(Stage<T> &st, int nblk, const int32_t *lo_g, con
 // before and then that block's triangle, while the other warps take the rest
 // of the columns: one barrier per block.
 template <typename T, bool kInv, int kNW>
-__device__ bool staged_backward_ahead(Stage<T> &st, int nblk, const int32_t *lo_g, const int64_t *ptr_g, int64_t base,
-                                      T *y, T *xb, int2 *meta, int tid) {
+__device__ bool staged_backward_ahead(Stage<T> &st, int nblk, const int2 *rows_g, T *y, T *xb, int2 *meta, int tid) {
   const int lane = tid & 31, w = tid >> 5;
   // the forward sweep left blocks nblk-1 and nblk-2, and their row tables
   bool late = false;
   if (w == 0) {
     const int b = nblk - 1, r0 = st.blk[b].x;
     late = !stage_wait(st, b);
-    backward_triangle<T, kInv>(stage_block(st, b), r0, st.blk[b + 1].x - r0, meta + (b & 1) * kSB, y,
+    backward_triangle<T, kInv>(stage_block(st, b), r0, st.blk[b + 1].x - r0, table4(meta, b), y,
                                xb + (b & 1) * kSB, lane);
   }
   if (__syncthreads_or(late)) return false;
   for (int b = nblk - 1; b >= 1; b--) {
     const int r0 = st.blk[b].x, nb = st.blk[b + 1].x - r0, rp = st.blk[b - 1].x;
-    const int2 *m = meta + (b & 1) * kSB;
+    const int2 *m = table4(meta, b);
     const T *S = stage_block(st, b), *x = xb + (b & 1) * kSB;
     late = false;
-    int lo2 = 0, pr2 = 0;  // the row table of block b - 2
     if (w == 0) {
-      if (b >= 2) stage_row_meta(lo_g, ptr_g, base, st.blk[b - 2].x, st.blk[b - 1].x, lane, lo2, pr2);
+      if (b >= 2) rows_issue(st, rows_g, table4(meta, b - 2), b - 2, lane);
       backward_columns(S, m, x, y, nb, rp, r0, lane);
       __syncwarp();
       late = !stage_wait(st, b - 1);
-      backward_triangle<T, kInv>(stage_block(st, b - 1), rp, r0 - rp, meta + ((b - 1) & 1) * kSB, y,
+      backward_triangle<T, kInv>(stage_block(st, b - 1), rp, r0 - rp, table4(meta, b - 1), y,
                                  xb + ((b - 1) & 1) * kSB, lane);
+      rows_wait();
     } else {
       const int bmin = __reduce_min_sync(0xffffffffu, lane < nb ? m[lane].x : INT_MAX);
       for (int cb = bmin + 32 * (w - 1); cb < rp; cb += 32 * (kNW - 1)) backward_columns(S, m, x, y, nb, cb, rp, lane);
     }
     if (__syncthreads_or(late)) return false;
-    if (b >= 2) {
-      stage_issue(st, b - 2, tid);
-      if (w == 0) {
-        meta[(b & 1) * kSB + lane] = make_int2(lo2, pr2);
-        __syncwarp();
-      }
-    }
+    if (b >= 2) stage_issue(st, b - 2, tid);
   }
   return true;
 }
@@ -1234,8 +1223,7 @@ __global__ void __launch_bounds__(kAhead ? 32 * kAhead : 128)
     }
     if (rn <= p.ir_tol * bn) return;  // the same decision in every thread
   }
-  const int32_t *lo_g = p.env_lo + io;
-  const int64_t *ptr_g = ptr_all + io;
+  const int2 *rows_g = (kInv ? p.inv_row_tab : p.row_tab) + io;
   T *z = zstash + io;
   // L2: the forward sweep's blocks are read again by the backward sweep, the
   // backward sweep's reads are the last use
@@ -1243,18 +1231,18 @@ __global__ void __launch_bounds__(kAhead ? 32 * kAhead : 128)
   st.policy = l2_evict_last();
   bool ok;
   if constexpr (kAhead != 0)
-    ok = staged_forward_ahead<T, kInv, kAhead>(st, nblk, lo_g, ptr_g, base, y, meta, z, rectb, tid);
+    ok = staged_forward_ahead<T, kInv, kAhead>(st, nblk, rows_g, y, meta, z, rectb, tid);
   else
-    ok = staged_forward<T, kInv>(st, nblk, lo_g, ptr_g, base, y, meta, z, rectb, tid);
+    ok = staged_forward<T, kInv>(st, nblk, rows_g, y, meta, z, rectb, tid);
   if (ok) {
 #pragma unroll 4
     for (int c = tid; c < nI; c += nt) y[c] = z[c];
     __syncthreads();
     st.policy = l2_evict_first();
     if constexpr (kAhead != 0)
-      ok = staged_backward_ahead<T, kInv, kAhead>(st, nblk, lo_g, ptr_g, base, y, rectb, meta, tid);
+      ok = staged_backward_ahead<T, kInv, kAhead>(st, nblk, rows_g, y, rectb, meta, tid);
     else
-      ok = staged_backward<T, kInv>(st, nblk, lo_g, ptr_g, base, y, rectb, meta, tid);
+      ok = staged_backward<T, kInv>(st, nblk, rows_g, y, rectb, meta, tid);
   }
   // every copy issued into this CTA's shared memory has landed before it exits
   stage_drain(st);
@@ -1265,6 +1253,14 @@ __global__ void __launch_bounds__(kAhead ? 32 * kAhead : 128)
     if (accumulate) x = cadd(xout[io + c], x);
     xout[io + c] = x;
   }
+}
+
+// The sweeps' row tables: per row its first column and the position of its
+// entries in its subdomain's.
+__global__ void row_table_kernel(DevProblem p, const int64_t *__restrict__ ptr, int2 *__restrict__ tab) {
+  const int s = p.sub_order[blockIdx.x];
+  const int64_t i0 = p.int_off[s], i1 = p.int_off[s + 1];
+  for (int64_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) tab[i] = make_int2(p.env_lo[i], (int)(ptr[i] - ptr[i0]));
 }
 
 // The block-inverse layout of one subdomain's factor, one warp per
@@ -1922,8 +1918,8 @@ void launch_staged_sweep(const DevProblem &p, int mode, const double2 *rhs, doub
 
 template <bool kInv>
 void launch_staged(const DevProblem &p, int mode, bool fp32, cudaStream_t stream) {
-  const StageLayout lay = kInv ? stage_layout(p.max_interior, p.inv_max_blocks, p.inv_cap, fp32)
-                               : stage_layout(p.max_interior, p.max_blocks, p.stage_cap, fp32);
+  const StageLayout lay = kInv ? stage_layout(p.max_interior, p.inv_max_blocks, p.inv_cap, fp32, p.stage_ahead)
+                               : stage_layout(p.max_interior, p.max_blocks, p.stage_cap, fp32, p.stage_ahead);
   double2 *rhs = fp32 ? p.B : p.Y;
   // one thread per row for both products: their rows are short (a few to a
   // few tens of entries) and the loads of several entries in flight per
@@ -1965,8 +1961,8 @@ void launch_subsolve(const DevProblem &p, int mode, bool fp32, cudaStream_t stre
     subsolve_kernel<false><<<nb, kThreads, 0, stream>>>(p, mode);
 }
 
-size_t subsolve_staged_smem_bytes(int max_interior, int max_blocks, int cap, bool fp32) {
-  return stage_layout(max_interior, max_blocks, cap, fp32).total;
+size_t subsolve_staged_smem_bytes(int max_interior, int max_blocks, int cap, bool fp32, bool ahead) {
+  return stage_layout(max_interior, max_blocks, cap, fp32, ahead).total;
 }
 
 // The dynamic shared-memory limit of a kernel is process-wide (per device):
@@ -2000,8 +1996,11 @@ int configure_sweep(int slot, size_t smem) {
   const void *const f[kSweepVariants] = {(const void *)subsolve_staged_kernel<T, kInv, 0>,
                                          (const void *)subsolve_staged_kernel<T, kInv, 4>,
                                          (const void *)subsolve_staged_kernel<T, kInv, 8>};
+  if (smem > 227 * 1024) return -1;
+  // the sweeps that take rows ahead hold two more row tables
+  const size_t ahead = std::min<size_t>(smem + 2 * kSB * 8, 227 * 1024);
   for (int k = 0; k < kSweepVariants; k++)
-    if (const int rc = raise_smem_limit(f[k], slot + k, smem)) return rc;
+    if (const int rc = raise_smem_limit(f[k], slot + k, k == 0 ? smem : ahead)) return rc;
   return 0;
 }
 }  // namespace
@@ -2012,6 +2011,10 @@ int configure_subsolve_staged(size_t smem, bool fp32) {
 
 int configure_subsolve_inv(size_t smem, bool fp32) {
   return fp32 ? configure_sweep<float2, true>(kSlotInv32, smem) : configure_sweep<double2, true>(kSlotInv64, smem);
+}
+
+void launch_row_table(const DevProblem &p, const int64_t *ptr, int2 *tab, cudaStream_t stream) {
+  if (p.nsub > 0) row_table_kernel<<<p.nsub, 128, 0, stream>>>(p, ptr, tab);
 }
 
 void launch_inv_relayout(const DevProblem &p, const double2 *L64, bool fp32, cudaStream_t stream) {

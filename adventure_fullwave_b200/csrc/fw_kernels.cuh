@@ -95,6 +95,7 @@ struct DevProblem {
   // staged solve on the block-inverse layout (kSolveInv): per block of rows,
   // the rows' entries left of the block, then N = (I + L_bb)^-1 - I strictly
   // lower and row-major (row t at t(t-1)/2), then the block's pivots 1/d
+  const int2 *row_tab, *inv_row_tab;  // sum nI: (first column, position in the subdomain's entries), staged sweeps
   const int64_t *inv_ptr;        // sum nI: position of each row's left entries in Linv
   const double2 *Linv64;
   const float2 *Linv32;
@@ -202,11 +203,12 @@ void launch_to_fp32(int64_t n, const double2 *src, float2 *dst, cudaStream_t str
 void launch_subsolve(const DevProblem &p, int mode, bool fp32, cudaStream_t stream);
 size_t subsolve_smem_bytes(int max_interior, int max_iface, bool fp32);
 int configure_subsolve(size_t smem, bool fp32);
-size_t subsolve_staged_smem_bytes(int max_interior, int max_blocks, int cap, bool fp32);
+size_t subsolve_staged_smem_bytes(int max_interior, int max_blocks, int cap, bool fp32, bool ahead);
 int configure_subsolve_staged(size_t smem, bool fp32);
 int configure_subsolve_inv(size_t smem, bool fp32);
 // the block-inverse layout (DevProblem inv_*) from the FP64 factor L64 in the
 // envelope layout, in FP32 (Linv32) or FP64 (Linv64)
+void launch_row_table(const DevProblem &p, const int64_t *ptr, int2 *tab, cudaStream_t stream);
 void launch_inv_relayout(const DevProblem &p, const double2 *L64, bool fp32, cudaStream_t stream);
 // Raises (never lowers) the dynamic shared-memory limit of kernel `func` on
 // the current device; `slot` names the kernel.

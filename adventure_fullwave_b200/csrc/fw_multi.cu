@@ -136,29 +136,37 @@ constexpr int kSweepThreads = 256; // 32 rows (or columns) x kRS sources at a ti
 
 struct MultiLayout {
   size_t y, buf0, buf1, dinv, meta, rect, bar, blk, total;
+  int tight;  // one row table, no 1/d in shared memory
 };
 
-__host__ __device__ inline MultiLayout multi_layout(int max_interior, int max_blocks, int cap, bool fp32) {
+inline MultiLayout multi_layout(int max_interior, int max_blocks, int cap, bool fp32) {
   const size_t es = fp32 ? 8 : 16;
   MultiLayout l;
-  size_t o = 0;
-  l.y = o;
-  o += a16((size_t)max_interior * kRS * es);
-  l.buf0 = o;
-  o += a16((size_t)cap * es);
-  l.buf1 = o;
-  o += a16((size_t)cap * es);
-  l.dinv = o;
-  o += a16((size_t)max_interior * es);
-  l.meta = o;
-  o += 32 * 8;
-  l.rect = o;
-  o += a16((size_t)32 * kRS * es);
-  l.bar = o;
-  o += 32;
-  l.blk = o;
-  o += a16(((size_t)max_blocks + 1) * 8);
-  l.total = o;
+  // the largest subdomains (FP64: interiors over about 1,330 DOFs, up to
+  // about 1,500) leave no room for the pivots and a second row table: their
+  // sweeps read the pivots again from the factor and wait for each block's
+  // table
+  for (l.tight = 0; l.tight < 2; l.tight++) {
+    size_t o = 0;
+    l.y = o;
+    o += a16((size_t)max_interior * kRS * es);
+    l.buf0 = o;
+    o += a16((size_t)cap * es);
+    l.buf1 = o;
+    o += a16((size_t)cap * es);
+    l.dinv = o;
+    if (!l.tight) o += a16((size_t)max_interior * es);
+    l.meta = o;
+    o += (l.tight ? 1 : 2) * 32 * 8;
+    l.rect = o;
+    o += a16((size_t)32 * kRS * es);
+    l.bar = o;
+    o += 16;
+    l.blk = o;
+    o += a16(((size_t)max_blocks + 1) * 8);
+    l.total = o;
+    if (l.tight || o <= 227 * 1024) break;
+  }
   return l;
 }
 
@@ -200,7 +208,8 @@ __global__ void __launch_bounds__(kSweepThreads, 2) multi_sweep_kernel(MultiProb
   if (nI == 0 || nblk <= 0) return;
   T *__restrict__ y = (T *)(smem_raw + lay.y);
   T *__restrict__ dinv = (T *)(smem_raw + lay.dinv);
-  int2 *meta = (int2 *)(smem_raw + lay.meta);
+  int2 *rows = (int2 *)(smem_raw + lay.meta);
+  const int tabs = lay.tight ? 0 : 1;  // mask of the row tables
   T *__restrict__ rect = (T *)(smem_raw + lay.rect);
   int2 *blk = (int2 *)(smem_raw + lay.blk);
   Stage<T> st;
@@ -221,30 +230,28 @@ __global__ void __launch_bounds__(kSweepThreads, 2) multi_sweep_kernel(MultiProb
   const int64_t g0 = io * kR + part * kRS;
   for (int e = tid; e < nI * kRS; e += nt) y[e] = from_d2<T>(rhs[g0 + (int64_t)(e / kRS) * kR + (e % kRS)]);
   __syncthreads();
-  const int32_t *lo_g = p.env_lo + io;
-  const int64_t *ptr_g = p.env_ptr + io;
+  const int2 *rows_g = p.row_tab + io;
   const int r = tid % kRS, row = tid / kRS;  // of the (row, source) passes
   constexpr int kRows = nt / kRS;
 
   // forward
   bool ok = true;
-  int nlo, npr;
   stage_issue(st, 0, tid);
-  stage_row_meta(lo_g, ptr_g, base, blk[0].x, blk[1].x, lane, nlo, npr);
+  if (warp == 0) rows_issue(st, rows_g, rows, 0, lane);
   for (int b = 0; b < nblk; b++) {
     const int r0 = blk[b].x, nb = blk[b + 1].x - r0;
-    const int my_lo = nlo, my_pr = npr;
-    if (warp == 0) meta[lane] = make_int2(nlo, npr);
-    if (b + 1 < nblk) {
-      stage_issue(st, b + 1, tid);
-      stage_row_meta(lo_g, ptr_g, base, blk[b + 1].x, blk[b + 2].x, lane, nlo, npr);
-    }
+    const int2 *meta = rows + (b & tabs) * 32;
+    const bool next = b + 1 < nblk;
+    if (next) stage_issue(st, b + 1, tid);
+    if (warp == 0) rows_wait();
     const bool late = !stage_wait(st, b);
     if (__syncthreads_or(late)) {
       ok = false;
       break;
     }
+    if (warp == 0 && next && tabs) rows_issue(st, rows_g, rows + ((b + 1) & tabs) * 32, b + 1, lane);
     const T *S = ((b & 1) ? st.buf1 : st.buf0) - stage_a0(st, b);
+    const int my_lo = meta[lane].x, my_pr = meta[lane].y;
     // entries left of the block
     for (int t = row; t < nb; t += kRows) {
       const int2 mt = meta[t];
@@ -330,35 +337,41 @@ __global__ void __launch_bounds__(kSweepThreads, 2) multi_sweep_kernel(MultiProb
       }
       if (in) {
         y[(r0 + lane) * kRS + q] = val;
-        if (q == 0) dinv[r0 + lane] = mine[lane];  // 1/d on the diagonal
+        if (q == 0 && tabs) dinv[r0 + lane] = mine[lane];  // 1/d on the diagonal
+      }
+    }
+    __syncthreads();
+    if (warp == 0 && next && !tabs) rows_issue(st, rows_g, rows, b + 1, lane);
+  }
+  if (ok) {
+    if (tabs) {
+      for (int e = tid; e < nI * kRS; e += nt) y[e] = cmul_rn(dinv[e / kRS], y[e]);
+    } else {
+      for (int e = tid; e < nI * kRS; e += nt) {
+        const int i = e / kRS;
+        const int2 t = rows_g[i];
+        y[e] = cmul_rn(st.L[t.y + i - t.x], y[e]);
       }
     }
     __syncthreads();
   }
-  if (ok) {
-    for (int e = tid; e < nI * kRS; e += nt) y[e] = cmul_rn(dinv[e / kRS], y[e]);
-    __syncthreads();
-  }
 
   // backward
-  if (ok) stage_row_meta(lo_g, ptr_g, base, blk[nblk - 1].x, blk[nblk].x, lane, nlo, npr);
   for (int b = nblk - 1; b >= 0 && ok; b--) {
     const int r0 = blk[b].x, nb = blk[b + 1].x - r0;
-    const int my_lo = nlo;
-    int bmin = lane < nb ? nlo : INT_MAX;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) bmin = min(bmin, __shfl_xor_sync(0xffffffffu, bmin, o));
-    if (warp == 0) meta[lane] = make_int2(nlo, npr);
-    // the forward sweep left blocks nblk-1 and nblk-2 in the buffers
-    if (b >= 1) {
-      if (b - 1 < nblk - 2) stage_issue(st, b - 1, tid);
-      stage_row_meta(lo_g, ptr_g, base, blk[b - 1].x, blk[b].x, lane, nlo, npr);
-    }
+    const int2 *meta = rows + (b & tabs) * 32;
+    // the forward sweep left blocks nblk-1 and nblk-2 in the buffers, and their row tables
+    const bool next = b >= 1 && b - 1 < nblk - 2;
+    if (next) stage_issue(st, b - 1, tid);
+    if (warp == 0) rows_wait();
     const bool late = !stage_wait(st, b);
     if (__syncthreads_or(late)) {
       ok = false;
       break;
     }
+    if (warp == 0 && next && tabs) rows_issue(st, rows_g, rows + ((b - 1) & tabs) * 32, b - 1, lane);
+    const int my_lo = meta[lane].x;
+    const int bmin = __reduce_min_sync(0xffffffffu, lane < nb ? my_lo : INT_MAX);
     const T *S = ((b & 1) ? st.buf1 : st.buf0) - stage_a0(st, b);
     // the triangle from the last row, lanes over the block's columns
     for (int q = warp; q < kRS; q += nw) {
@@ -409,6 +422,7 @@ __global__ void __launch_bounds__(kSweepThreads, 2) multi_sweep_kernel(MultiProb
       if (in) y[c * kRS + r] = yc;
     }
     __syncthreads();
+    if (warp == 0 && b >= 1 && !tabs) rows_issue(st, rows_g, rows, b - 1, lane);
   }
   // every copy issued into this CTA's shared memory has landed before it exits
   stage_drain(st);

@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 
 from adventure_fullwave_b200 import hddm, meshgen
+from helpers import rel_l2
 
 pytestmark = pytest.mark.gpu
 
@@ -22,3 +23,19 @@ def test_same_bits_for_every_share(n, leaf, precision, kernel):
         got.append((np.asarray(x), r.iterations))
     for x, its in got[1:]:
         assert its == got[0][1] and np.array_equal(x, got[0][0], equal_nan=True)
+
+
+@pytest.mark.parametrize("n,leaf", [(8, 1600), (9, 1500)])
+def test_batched_sources_on_the_largest_subdomains(n, leaf):
+    """FP64 batched sources where a subdomain of 1,451 interior DOFs leaves no
+    shared memory for the pivots and a second row table, and where all of at
+    most 1,094 leave it: each source against the one-source solve, 1e-8."""
+    model = meshgen.make_model("w", n=n, size=1.0, npml=1, layers=2, nleaves=None, leaf_cap=leaf, jitter=(0.3, 0.7),
+                               seed=5, nsources=3)
+    meshgen.round_trip_material(model)
+    with hddm.HddmSolver(model, hddm_eps=1e-10, hddm_max_loop=20000) as s:
+        res = s.solve_multi([0, 1, 2])
+        xs = [s.edge_solution_multi(k) for k in range(3)]
+        for k in range(3):
+            s.resolve(k)
+            assert res[k].converged and rel_l2(xs[k], s.edge_solution()) <= 1e-8
