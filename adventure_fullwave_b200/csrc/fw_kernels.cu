@@ -204,19 +204,19 @@ __global__ void factor_kernel(int32_t nsub, const int32_t *__restrict__ sub_orde
 // lane: the butterfly's first two steps are then sums within a lane.  Rows
 // are read through L1; the pivots and the row table stay in shared memory.
 constexpr int kFB = 16;
-constexpr int kFactorThreads = 256;
 
 size_t factor_block_smem(int max_interior) { return (size_t)max_interior * 24; }
 
-__global__ void __launch_bounds__(kFactorThreads) factor_block_kernel(const int32_t *__restrict__ sub_order,
-                                                                     const int64_t *__restrict__ int_off,
-                                                                     const int32_t *__restrict__ env_lo,
-                                                                     const int64_t *__restrict__ env_ptr, double2 *L,
-                                                                     int32_t *status) {
+template <int kThr>
+__global__ void __launch_bounds__(kThr) factor_block_kernel(const int32_t *__restrict__ sub_order,
+                                                           const int64_t *__restrict__ int_off,
+                                                           const int32_t *__restrict__ env_lo,
+                                                           const int64_t *__restrict__ env_ptr, double2 *L,
+                                                           int32_t *status) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int s = sub_order[blockIdx.x];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, j8 = lane & 7;
-  constexpr int kGroups = kFactorThreads / 8;
+  constexpr int kGroups = kThr / 8;
   const int64_t o = int_off[s];
   const int nI = (int)(int_off[s + 1] - o);
   if (nI == 0) return;
@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(kFactorThreads) factor_block_kernel(const int3
   int32_t *pr = lo + nI;                // row start less its first column: entry (i, k) at pr[i] + k
   const int64_t base = env_ptr[o];
   double2 *B = L + base;
-  for (int i = tid; i < nI; i += kFactorThreads) {
+  for (int i = tid; i < nI; i += kThr) {
     lo[i] = env_lo[o + i];
     pr[i] = (int32_t)(env_ptr[o + i] - base) - lo[i];
   }
@@ -1256,8 +1256,8 @@ __global__ void row_table_kernel(DevProblem p, const int64_t *__restrict__ ptr, 
   for (int64_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) tab[i] = make_int2(p.env_lo[i], (int)(ptr[i] - ptr[i0]));
 }
 
-// The block-inverse layout of one subdomain's factor, one warp per
-// subdomain, block by block.  For the block of rows r0..r0+nb-1:
+// The block-inverse layout of one subdomain's factor, block by block, the
+// blocks shared by the warps of blockIdx.y.  For the block of rows r0..r0+nb-1:
 //   - each row's entries left of the block (columns lo..r0-1), copied;
 //   - N = (I + L_bb)^-1 - I, strictly lower, row-major (row i at i(i-1)/2),
 //     where L_bb is the block's own part of the unit lower factor; row by
@@ -1269,13 +1269,12 @@ __global__ void row_table_kernel(DevProblem p, const int64_t *__restrict__ ptr, 
 template <typename T>
 __global__ void __launch_bounds__(32) inv_relayout_kernel(DevProblem p, const double2 *__restrict__ L64, T *out) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  double2 *M = (double2 *)smem_raw;  // [32][33]: L_bb
-  double2 *Nd = M + 32 * 33;         // [32][33]: N
+  double2 *M = (double2 *)smem_raw;  // [32][33]: L_bb, its rows turned into N's one after another
   const int s = p.sub_order[blockIdx.x], lane = threadIdx.x;  // the subdomains this context solves
   const int64_t io = p.int_off[s];
   const int b0 = p.inv_blk_off[s];
   const int nblk = p.inv_blk_off[s + 1] - b0 - 1;
-  for (int b = 0; b < nblk; b++) {
+  for (int b = blockIdx.y; b < nblk; b += gridDim.y) {
     const int r0 = p.inv_blk_tab[b0 + b].x, nb = p.inv_blk_tab[b0 + b + 1].x - r0;
     int lo = r0;
     int64_t ep = 0, ip = 0;
@@ -1293,17 +1292,20 @@ __global__ void __launch_bounds__(32) inv_relayout_kernel(DevProblem p, const do
     }
     __syncwarp();
     for (int i = 1; i < nb; i++) {
+      double2 acc = cz();
       if (lane < i) {
-        double2 acc = M[i * 33 + lane];
-        for (int k = lane + 1; k < i; k++) acc = cmac(acc, M[i * 33 + k], Nd[k * 33 + lane]);
-        Nd[i * 33 + lane] = make_double2(-acc.x, -acc.y);  // lane j reads only its own column of N
+        acc = M[i * 33 + lane];
+        for (int k = lane + 1; k < i; k++) acc = cmac(acc, M[i * 33 + k], M[k * 33 + lane]);
       }
+      __syncwarp();  // every lane has read row i
+      if (lane < i) M[i * 33 + lane] = make_double2(-acc.x, -acc.y);
+      __syncwarp();
     }
     const int lo_l = __shfl_sync(0xffffffffu, lo, nb - 1);
     const int64_t ip_l = __shfl_sync(0xffffffffu, ip, nb - 1);
     const int64_t tri0 = ip_l + max(0, r0 - lo_l);
     for (int i = 1; i < nb; i++)
-      if (lane < i) out[tri0 + ((i * (i - 1)) >> 1) + lane] = from_d2<T>(Nd[i * 33 + lane]);
+      if (lane < i) out[tri0 + ((i * (i - 1)) >> 1) + lane] = from_d2<T>(M[i * 33 + lane]);
     if (lane < nb) out[tri0 + ((nb * (nb - 1)) >> 1) + lane] = from_d2<T>(L64[ep + (r0 + lane - lo)]);
     __syncwarp();  // M and N are rewritten for the next block
   }
@@ -1881,10 +1883,20 @@ void launch_factor(const DevProblem &p, const int64_t *int_off, const int32_t *e
                    double2 *L, int32_t *status, cudaStream_t stream) {
   if (p.nsub <= 0) return;
   // one CTA per subdomain while its row table fits in shared memory (9,600
-  // interior DOFs)
+  // interior DOFs).  The rows below a block are shared by the CTA's eight-lane
+  // groups: where there are few subdomains, an SM's threads all go to the one
+  // or two (four) that it has.  Setup of a solve with 256 threads and so: 59
+  // subdomains of up to 600 elements 2.14 and 1.64 ms, 58 of up to 1200 8.3 and
+  // 5.4, 551 of up to 600 3.20 and 2.85.
   const size_t smem = factor_block_smem(p.max_interior);
-  if (raise_smem_limit((const void *)factor_block_kernel, kSlotFactor, smem) == 0) {
-    factor_block_kernel<<<p.nsub, kFactorThreads, smem, stream>>>(p.sub_order, int_off, env_lo, env_ptr, L, status);
+  const int per_sm = (p.nsub + kSms - 1) / kSms;
+  const auto kernel = per_sm <= 2   ? factor_block_kernel<1024>
+                      : per_sm <= 4 ? factor_block_kernel<512>
+                                    : factor_block_kernel<256>;
+  const int threads = per_sm <= 2 ? 1024 : per_sm <= 4 ? 512 : 256;
+  const int slot = per_sm <= 2 ? kSlotFactor1024 : per_sm <= 4 ? kSlotFactor512 : kSlotFactor;
+  if (raise_smem_limit((const void *)kernel, slot, smem) == 0) {
+    kernel<<<p.nsub, threads, smem, stream>>>(p.sub_order, int_off, env_lo, env_ptr, L, status);
     return;
   }
   factor_kernel<<<blocks_for((int64_t)p.nsub * 32, kThreads), kThreads, 0, stream>>>(p.nsub, p.sub_order, int_off,
@@ -2012,11 +2024,12 @@ void launch_row_table(const DevProblem &p, const int64_t *ptr, int2 *tab, cudaSt
 
 void launch_inv_relayout(const DevProblem &p, const double2 *L64, bool fp32, cudaStream_t stream) {
   if (p.nsub <= 0) return;
-  constexpr size_t smem = 2 * 32 * 33 * sizeof(double2);
+  constexpr size_t smem = 32 * 33 * sizeof(double2);
+  const dim3 grid(p.nsub, 8);
   if (fp32)
-    inv_relayout_kernel<float2><<<p.nsub, 32, smem, stream>>>(p, L64, (float2 *)(void *)p.Linv32);
+    inv_relayout_kernel<float2><<<grid, 32, smem, stream>>>(p, L64, (float2 *)(void *)p.Linv32);
   else
-    inv_relayout_kernel<double2><<<p.nsub, 32, smem, stream>>>(p, L64, (double2 *)(void *)p.Linv64);
+    inv_relayout_kernel<double2><<<grid, 32, smem, stream>>>(p, L64, (double2 *)(void *)p.Linv64);
 }
 
 int subsolve_launches(const DevProblem &p, bool fp32) {

@@ -212,6 +212,8 @@ void launch_row_table(const DevProblem &p, const int64_t *ptr, int2 *tab, cudaSt
 void launch_inv_relayout(const DevProblem &p, const double2 *L64, bool fp32, cudaStream_t stream);
 // Raises (never lowers) the dynamic shared-memory limit of kernel `func` on
 // the current device; `slot` names the kernel.
+// SMs of a B200: the rules that must give the same choice on every run count with this
+constexpr int kSms = 148;
 // Slots of the process-wide dynamic shared-memory limits (raise_smem_limit):
 // one per kernel instantiation that runs above the 48 KB default.
 constexpr int kSweepVariants = 3;  // the plain staged sweep; with the rows taken ahead by 4 and by 8 warps
@@ -225,6 +227,8 @@ enum SmemSlot {
   kSlotMulti32,
   kSlotMulti64,
   kSlotFactor,
+  kSlotFactor512,
+  kSlotFactor1024,
   kSmemSlots
 };
 int raise_smem_limit(const void *func, int slot, size_t smem);
