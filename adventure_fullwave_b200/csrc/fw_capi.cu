@@ -1030,7 +1030,7 @@ static int build_row_table(fwgpu_context *c, const int64_t *d_ptr, const int2 **
 // (the rows' entries left of the block, the block's N = (I + L_bb)^-1 - I as
 // a dense strict lower triangle, and its pivots) fit one staging buffer of
 // `cap` elements, each subdomain's elements from a 16-byte boundary.
-static int build_inv_blocks(fwgpu_context *c, int cap) {
+static int build_inv_blocks(fwgpu_context *c, int cap, bool optional) {
   const fw::Plan &p = c->p;
   const int nsub = c->m.nsub;
   const bool fp32 = c->opts.precision == FWGPU_PREC_FP32_IR;
@@ -1080,14 +1080,16 @@ static int build_inv_blocks(fwgpu_context *c, int cap) {
     c->inv_ok = false;
     return FWGPU_OK;
   }
+  // padding: bulk copies of a block may read up to 16 bytes past its end
+  const int rc = fp32 ? c->alloc(&c->d_Linv32, pos + 64) : c->alloc(&c->d_Linv64, pos + 64);
+  if (rc != FWGPU_OK && optional) {  // no room for the copy: the staged sweep
+    (void)cudaGetLastError();
+    return FWGPU_OK;
+  }
+  FW_TRY(rc);
   FW_TRY(c->upload(&c->d_inv_blk_off, boff));
   FW_TRY(c->upload(&c->d_inv_blk_tab, btab));
   FW_TRY(c->upload(&c->d_inv_ptr, iptr));
-  // padding: bulk copies of a block may read up to 16 bytes past its end
-  if (fp32)
-    FW_TRY(c->alloc(&c->d_Linv32, pos + 64));
-  else
-    FW_TRY(c->alloc(&c->d_Linv64, pos + 64));
   c->inv_len = pos;
   c->dp.inv_ptr = c->d_inv_ptr;
   FW_TRY(build_row_table(c, c->d_inv_ptr, &c->dp.inv_row_tab));
@@ -1133,6 +1135,37 @@ static int setup_stage(fwgpu_context *c) {
                               nullptr));
   }
   return FWGPU_OK;
+}
+
+// Staging capacity of the block-inverse sweep.  Every block costs a sweep the
+// same barriers and the same full products with N, so it wants blocks of many
+// rows; larger buffers leave fewer subdomains on an SM.
+//   - Up to six subdomains per SM, 64 rows of the average length (the longest
+//     rows come last), as long as an SM holds two subdomains, or its one.
+//     Per phase: 59 subdomains of up to 600 elements FP64 102 us with 1024
+//     elements, 72 with 3072; 58 of up to 1200 FP64 316, and 155 with 4096,
+//     FP32 313, and 228 with 8192; 551 of up to 600 FP64 164, and 111 with
+//     2560; 636 of up to 1200 FP64 504, 298 with 2560 (two per SM) and 427
+//     with 3072 (one).
+//   - More, FP64, 22 rows: 5093 of up to 900 1297 us with 1024, 1257 with
+//     1536; 1463 of up to 1200 743 us with 1024, 613 with
+//     1536, 659 with 2048; 1654 of up to 600 244 with 1024, 252 with 1536;
+//     3811 of up to 200 141 and 155.  FP32 keeps the staged kernel's: 2253 of
+//     up to 1000 take 849, 814, 812 and 829 us with 1536, 2048, 2560, 3072.
+static int inv_stage_cap(const fwgpu_context *c) {
+  const bool fp32 = c->opts.precision == FWGPU_PREC_FP32_IR;
+  const int64_t rows = c->p.sub_int_off[c->m.nsub];
+  const int per_sm = (c->m.nsub + fw::kSms - 1) / fw::kSms;
+  const int64_t want = per_sm <= 6 ? 64 : fp32 ? 0 : 22;
+  int cap = c->dp.stage_cap;
+  for (int k = 3; k <= 8 && cap * rows < want * c->nlen_int; k++) {
+    const int next = (c->dp.stage_cap * k / 2) & ~7;
+    const size_t smem = fw::subsolve_staged_smem_bytes(c->p.max_interior, c->dp.max_blocks, next, fp32, true);
+    // an SM's 228 KB, of which each CTA takes 1 KB and its static part besides
+    if (smem > 226 * 1024 || (int)(228 * 1024 / (smem + 1280)) < std::min(2, per_sm)) break;
+    cap = next;
+  }
+  return cap;
 }
 
 // Times the candidate subdomain-solve kernels on the factors just computed
@@ -1244,15 +1277,20 @@ int fwgpu_solve_dom_1st(fwgpu_context *c) {
     FW_TRY(setup_stage(c));
     if (c->opts.solve_kernel == FWGPU_SOLVE_WARP && !c->warp_ok)
       return set_error(FWGPU_ERR_ARG, "staged solve kernel: subdomains too large for shared memory");
-    // the block-inverse layout: asked for, or AUTO with FP32 factors, where
-    // it is the faster sweep (C2 12 %, C3 3 %; with FP64 factors the two
-    // sweeps take the same time)
+    // the block-inverse layout: asked for, or AUTO while the second copy of the
+    // factor that it takes is small beside the memory (FP32 factors are half as
+    // large).  The triangles' chains are what few subdomains wait for, and with
+    // many its blocks of more rows save: per iteration, staged and so, 59
+    // subdomains of up to 600 elements FP64 125 and 81 us, 58 of up to 1200 318
+    // and 165, 1463 of up to 1200 758 and 644, 3811 of up to 200 177 and 166,
+    // 1654 of up to 600 277 and 268, 5093 of up to 900 1394 and 1337.
     const bool fp32 = c->opts.precision == FWGPU_PREC_FP32_IR;
-    const bool inv = c->opts.solve_kernel == FWGPU_SOLVE_BLOCKINV || (c->opts.solve_kernel == FWGPU_SOLVE_AUTO && fp32);
-    if (inv && c->warp_ok) {
-      // staging capacity: the caller's, else the staged kernel's, whose rule
-      // was also the fastest of 1, 1.5 and 2 times it for this layout
-      FW_TRY(build_inv_blocks(c, c->opts.stage_cap > 0 ? c->opts.stage_cap : c->dp.stage_cap));
+    const bool any = c->opts.solve_kernel == FWGPU_SOLVE_AUTO;
+    const bool asked = c->opts.solve_kernel == FWGPU_SOLVE_BLOCKINV;
+    constexpr int64_t kInvCopyMax = (int64_t)4 << 30;  // bytes of FP64 factor
+    if (c->warp_ok && (asked || (any && (fp32 || pos * (int64_t)sizeof(double2) <= kInvCopyMax)))) {
+      const int cap = c->opts.stage_cap <= 0 ? inv_stage_cap(c) : any && !fp32 ? c->dp.stage_cap : c->opts.stage_cap;
+      FW_TRY(build_inv_blocks(c, cap, any && !fp32));
     }
     if (c->opts.solve_kernel == FWGPU_SOLVE_BLOCKINV && !c->inv_ok)
       return set_error(FWGPU_ERR_ARG, "block-inverse solve kernel: subdomains too large for shared memory");

@@ -39,3 +39,19 @@ def test_batched_sources_on_the_largest_subdomains(n, leaf):
         for k in range(3):
             s.resolve(k)
             assert res[k].converged and rel_l2(xs[k], s.edge_solution()) <= 1e-8
+
+
+@pytest.mark.parametrize("n,leaf", [(4, 7), (6, 110), (8, 4), (8, 600), (8, 1600)])
+@pytest.mark.parametrize("precision", ["fp64", "fp32_ir"])
+def test_auto_sweep_against_the_staged_one(n, leaf, precision):
+    """The timed choice's block-inverse sweep, at the capacities it takes for
+    one subdomain per SM, a few and many, against the staged sweep: both
+    converged to 1e-10, 1e-8 (FP32 with refinement 1e-6, as against the oracle)."""
+    model = meshgen.make_model("w", n=n, size=1.0, npml=1, layers=2, nleaves=None, leaf_cap=leaf, jitter=(0.3, 0.7),
+                               seed=5)
+    meshgen.round_trip_material(model)
+    kw = dict(hddm_eps=1e-10, hddm_max_loop=20000, precision=precision, ir_max_steps=2)
+    x, r = hddm.hddm_solver_CS(model, 0, **kw)
+    want, rw = hddm.hddm_solver_CS(model, 0, solve_kernel="warp", **kw)
+    assert r.solve_kernel == "blockinv" and r.converged and rw.converged
+    assert rel_l2(np.asarray(x), np.asarray(want)) <= (1e-8 if precision == "fp64" else 1e-6)
