@@ -1147,8 +1147,7 @@ static int setup_stage(fwgpu_context *c) {
 //     FP32 313, and 228 with 8192; 551 of up to 600 FP64 164, and 111 with
 //     2560; 636 of up to 1200 FP64 504, 298 with 2560 (two per SM) and 427
 //     with 3072 (one).
-//   - More, FP64, 22 rows: 5093 of up to 900 1297 us with 1024, 1257 with
-//     1536; 1463 of up to 1200 743 us with 1024, 613 with
+//   - More, FP64, 22 rows: 1463 of up to 1200 743 us with 1024, 613 with
 //     1536, 659 with 2048; 1654 of up to 600 244 with 1024, 252 with 1536;
 //     3811 of up to 200 141 and 155.  FP32 keeps the staged kernel's: 2253 of
 //     up to 1000 take 849, 814, 812 and 829 us with 1536, 2048, 2560, 3072.
@@ -1277,17 +1276,18 @@ int fwgpu_solve_dom_1st(fwgpu_context *c) {
     FW_TRY(setup_stage(c));
     if (c->opts.solve_kernel == FWGPU_SOLVE_WARP && !c->warp_ok)
       return set_error(FWGPU_ERR_ARG, "staged solve kernel: subdomains too large for shared memory");
-    // the block-inverse layout: asked for, or AUTO while the second copy of the
-    // factor that it takes is small beside the memory (FP32 factors are half as
-    // large).  The triangles' chains are what few subdomains wait for, and with
+    // the block-inverse layout: asked for, or AUTO with FP32 factors, or AUTO
+    // with FP64 factors up to 1 GiB.  The triangles' chains are what few subdomains wait for, and with
     // many its blocks of more rows save: per iteration, staged and so, 59
     // subdomains of up to 600 elements FP64 125 and 81 us, 58 of up to 1200 318
     // and 165, 1463 of up to 1200 758 and 644, 3811 of up to 200 177 and 166,
-    // 1654 of up to 600 277 and 268, 5093 of up to 900 1394 and 1337.
+    // 1654 of up to 600 277 and 268.  Above, the staged sweep: 5093 of up to
+    // 900 (1.7 GB) took 1394 and 1337, for a second copy of the factor and, on
+    // 350 iterations, a solution that moved by 2e-10 with the rounding.
     const bool fp32 = c->opts.precision == FWGPU_PREC_FP32_IR;
     const bool any = c->opts.solve_kernel == FWGPU_SOLVE_AUTO;
     const bool asked = c->opts.solve_kernel == FWGPU_SOLVE_BLOCKINV;
-    constexpr int64_t kInvCopyMax = (int64_t)4 << 30;  // bytes of FP64 factor
+    constexpr int64_t kInvCopyMax = (int64_t)1 << 30;  // bytes of FP64 factor
     if (c->warp_ok && (asked || (any && (fp32 || pos * (int64_t)sizeof(double2) <= kInvCopyMax)))) {
       const int cap = c->opts.stage_cap <= 0 ? inv_stage_cap(c) : any && !fp32 ? c->dp.stage_cap : c->opts.stage_cap;
       FW_TRY(build_inv_blocks(c, cap, any && !fp32));

@@ -155,7 +155,7 @@ typedef struct {
 } fwgpu_options;
 
 /* Batched subdomain-solve kernels.  AUTO runs the BLOCKINV kernel (the WARP
- * kernel where the FP64 factor is over 4 GiB) at the staging capacity that a
+ * kernel where the FP64 factor is over 1 GiB) at the staging capacity that a
  * rule on the envelope gives, and times 2, 4 and 8 warps per subdomain, which
  * sum in the same order; WARP also times its staging capacities, which
  * changes the order of the sums. */
