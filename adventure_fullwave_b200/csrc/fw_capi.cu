@@ -91,6 +91,7 @@ struct fwgpu_context {
   fw::DevProblem dp{};
   fw::CocgScalars *d_sc = nullptr;
   fw::CocgScalars *h_sc = nullptr;  // pinned
+  int32_t *h_post_bad = nullptr;    // pinned, after h_sc: the post step's kernel writes it
   double *d_hist = nullptr;
   cudaGraphExec_t graph = nullptr;
   int graph_iters = 0;
@@ -618,7 +619,8 @@ static int setup_device(fwgpu_context *c, const fwgpu_options *opts, fwgpu_conte
   FW_TRY(c->alloc(&dp.part, 8 * (size_t)nb));
   FW_TRY(c->alloc(&c->d_sc, 1));
   dp.sc = c->d_sc;
-  FW_CUDA(cudaMallocHost(&c->h_sc, sizeof(fw::CocgScalars)));
+  FW_CUDA(cudaMallocHost(&c->h_sc, sizeof(fw::CocgScalars) + sizeof(int32_t)));
+  c->h_post_bad = reinterpret_cast<int32_t *>(c->h_sc + 1);
   FW_TRY(c->alloc(&c->d_hist, (size_t)std::max(1, opts->hddm_max_loop) + 2));
   dp.hist = c->d_hist;
   dp.hist_cap = std::max(1, opts->hddm_max_loop) + 2;
@@ -1282,7 +1284,7 @@ int fwgpu_solve_dom_1st(fwgpu_context *c) {
     // subdomains of up to 600 elements FP64 125 and 81 us, 58 of up to 1200 318
     // and 165, 1463 of up to 1200 758 and 644, 3811 of up to 200 177 and 166,
     // 1654 of up to 600 277 and 268.  Above, the staged sweep: 5093 of up to
-    // 900 (1.7 GB) took 1394 and 1337, for a second copy of the factor and, on
+    // 900 (1.8 GB) took 1394 and 1337, for a second copy of the factor and, on
     // 350 iterations, a solution that moved by 2e-10 with the rounding.
     const bool fp32 = c->opts.precision == FWGPU_PREC_FP32_IR;
     const bool any = c->opts.solve_kernel == FWGPU_SOLVE_AUTO;
@@ -2024,18 +2026,19 @@ int fwgpu_post_em_E(fwgpu_context *c, const double *x, double *el_B, double *el_
       staged[k] = true;
     }
   }
-  FW_CUDA(cudaMemsetAsync(c->d_mesh_status + 2, 0, sizeof(int32_t), c->stream));
+  // the status stays in host memory that the kernel writes only for a
+  // degenerate element (every call waits for its stream below): with a memset
+  // and a copy back around the kernel 663,552 elements took 68 us, so 54
+  *c->h_post_bad = 0;
   fw::launch_post_em_E(nt, c->d_tv, c->d_te, c->d_crd, c->d_el_has_nu, c->d_el_sigma, c->m.omega, dx, out[0], out[1],
-                       out[2], c->d_mesh_status + 2, c->stream);
+                       out[2], c->h_post_bad, c->stream);
   c->launches += 1;
   FW_CUDA(cudaGetLastError());
   for (int k = 0; k < 3; k++)
     if (staged[k])
       FW_CUDA(cudaMemcpyAsync(user[k], out[k], 3 * nt * sizeof(double2), cudaMemcpyDeviceToHost, c->stream));
-  int32_t bad = 0;
-  FW_CUDA(cudaMemcpyAsync(&bad, c->d_mesh_status + 2, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
   FW_CUDA(cudaStreamSynchronize(c->stream));
-  if (bad) return set_error(FWGPU_ERR_MESH, "degenerate element in the post step");
+  if (*c->h_post_bad) return set_error(FWGPU_ERR_MESH, "degenerate element in the post step");
   return FWGPU_OK;
 }
 

@@ -399,7 +399,7 @@ __global__ void __launch_bounds__(kPostThreads, 4) post_em_E_kernel(int64_t nt, 
   if (t < nt) {
     double2 r[9];
     if (post_element(t, tet_vertices, tet_edges, crd, el_has_nu, el_sigma, s_nu, s_zero, xedge, r) && status)
-      atomicMax(status, 1);
+      *status = 1;  // the host's own memory, written for a degenerate element alone: no memset, no copy back
 #pragma unroll
     for (int k = 0; k < 3; k++) {
       stage[0][3 * threadIdx.x + k] = r[k];

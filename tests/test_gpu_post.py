@@ -80,3 +80,20 @@ def test_post_after_a_batched_solve_uses_the_source_last_read():
     want = oracle.post_em_E(m, x1)
     for g, w in zip(got, want):
         assert np.array_equal(g, w)
+
+
+def test_inverted_element_is_a_mesh_error():
+    """The post step's status of one inverted element (D <= 0), and that a
+    context of a sound mesh reports none before and after it."""
+    sound = meshgen.make_model("x", n=6, size=1.0, npml=1, nleaves=6, seed=1)
+    m = dataclasses.replace(sound, tets=sound.tets.copy(), tet_edges=sound.tet_edges.copy())
+    m.tets[5] = m.tets[5][[0, 2, 1, 3]]
+    m.tet_edges[5] = m.tet_edges[5][[1, 0, 2, 3, 5, 4]]
+    x = np.ones(m.n_edges, complex)
+    with hddm.HddmSolver(sound) as a, hddm.HddmSolver(m) as b:
+        want = a.post_em_E(x)
+        for _ in range(2):
+            with pytest.raises(_lib.FwgpuError) as e:
+                b.post_em_E(x)
+            assert e.value.code == _lib.ERR_MESH
+            assert all(np.array_equal(u, v) for u, v in zip(a.post_em_E(x), want))
