@@ -1179,9 +1179,9 @@ static int inv_stage_cap(const fwgpu_context *c) {
 // order of the sums, so AUTO keeps the default capacity (a rule on the
 // model's envelope, setup_stage) and times two and four warps per subdomain,
 // and four and eight with the next block's rows taken ahead, which share out
-// whole row groups and column chunks and so sum alike.  With FP32 factors AUTO
-// runs the block-inverse sweep (a rule, not a timed choice), with FP64 factors
-// the staged sweep.  The CTA kernel sums in another order and runs only when
+// whole row groups and column chunks and so sum alike.  AUTO
+// runs the block-inverse sweep where that layout was built (a rule on the
+// model, not a timed choice), else the staged sweep.  The CTA kernel sums in another order and runs only when
 // asked for.  An explicit WARP choice times the staging capacities too.
 static int tune_solve_kernel(fwgpu_context *c) {
   const bool fp32 = c->opts.precision == FWGPU_PREC_FP32_IR;
@@ -1201,7 +1201,7 @@ static int tune_solve_kernel(fwgpu_context *c) {
         if (c->opts.stage_warps == warps || (c->opts.stage_warps == 0 && !(any && warps == 1)))
           cand.push_back({variant, cap, warps, ahead});
   };
-  // AUTO runs the block-inverse sweep where it built that layout (FP32 factors)
+  // AUTO runs the block-inverse sweep where it built that layout
   const bool any_inv = any && c->inv_ok;
   if (any && c->warp_ok && !any_inv) sweeps(fw::kSolveWarp, c->dp.stage_cap);
   if (c->opts.solve_kernel == FWGPU_SOLVE_WARP && c->warp_ok)
@@ -1279,8 +1279,8 @@ int fwgpu_solve_dom_1st(fwgpu_context *c) {
     if (c->opts.solve_kernel == FWGPU_SOLVE_WARP && !c->warp_ok)
       return set_error(FWGPU_ERR_ARG, "staged solve kernel: subdomains too large for shared memory");
     // the block-inverse layout: asked for, or AUTO with FP32 factors, or AUTO
-    // with FP64 factors up to 1 GiB.  The triangles' chains are what few subdomains wait for, and with
-    // many its blocks of more rows save: per iteration, staged and so, 59
+    // with FP64 factors up to 1 GiB.  The triangles' chains are what few
+    // subdomains wait for, and with many its blocks of more rows save: per iteration, staged and so, 59
     // subdomains of up to 600 elements FP64 125 and 81 us, 58 of up to 1200 318
     // and 165, 1463 of up to 1200 758 and 644, 3811 of up to 200 177 and 166,
     // 1654 of up to 600 277 and 268.  Above, the staged sweep: 5093 of up to
