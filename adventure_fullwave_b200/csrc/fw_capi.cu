@@ -1179,10 +1179,11 @@ static int inv_stage_cap(const fwgpu_context *c) {
 // order of the sums, so AUTO keeps the default capacity (a rule on the
 // model's envelope, setup_stage) and times two and four warps per subdomain,
 // and four and eight with the next block's rows taken ahead, which share out
-// whole row groups and column chunks and so sum alike.  AUTO
-// runs the block-inverse sweep where that layout was built (a rule on the
-// model, not a timed choice), else the staged sweep.  The CTA kernel sums in another order and runs only when
-// asked for.  An explicit WARP choice times the staging capacities too.
+// whole row groups and column chunks and so sum alike.  AUTO runs the
+// block-inverse sweep where that layout was built (a rule on the model, not a
+// timed choice), else the staged sweep.  The CTA kernel sums in another order
+// and runs only when asked for.  An explicit WARP choice times the staging
+// capacities too.
 static int tune_solve_kernel(fwgpu_context *c) {
   const bool fp32 = c->opts.precision == FWGPU_PREC_FP32_IR;
   struct Cand {
