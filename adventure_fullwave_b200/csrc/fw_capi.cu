@@ -1078,7 +1078,7 @@ static int build_inv_blocks(fwgpu_context *c, int cap, bool optional) {
   }
   boff[nsub] = (int32_t)btab.size();
   const size_t smem = fw::subsolve_staged_smem_bytes(max_nI, max_blocks, cap, fp32, false);
-  if (smem > 227 * 1024 || fw::configure_subsolve_inv(smem, fp32) != 0) {
+  if (smem > fw::subsolve_staged_smem_max(false) || fw::configure_subsolve_inv(smem, fp32, false) != 0) {
     c->inv_ok = false;
     return FWGPU_OK;
   }
@@ -1101,7 +1101,8 @@ static int build_inv_blocks(fwgpu_context *c, int cap, bool optional) {
   c->dp.Linv32 = c->d_Linv32;
   c->dp.inv_max_blocks = max_blocks;
   c->dp.inv_cap = cap;
-  c->inv_ahead_ok = fw::subsolve_staged_smem_bytes(max_nI, max_blocks, cap, fp32, true) <= 227 * 1024;
+  const size_t ahead = fw::subsolve_staged_smem_bytes(max_nI, max_blocks, cap, fp32, true);
+  c->inv_ahead_ok = ahead <= fw::subsolve_staged_smem_max(true) && fw::configure_subsolve_inv(ahead, fp32, true) == 0;
   c->inv_ok = true;
   return FWGPU_OK;
 }
@@ -1117,20 +1118,23 @@ static int setup_stage(fwgpu_context *c) {
   if (c->opts.stage_cap > 0) cand = {c->opts.stage_cap};
   c->stage_caps.clear();
   c->stage_ahead_caps.clear();
-  size_t smem_max = 0;
+  size_t smem_max = 0, ahead_max = 0;
   for (int cap : cand) {
     cap = std::max(cap, min_cap);
     if (std::find(c->stage_caps.begin(), c->stage_caps.end(), cap) != c->stage_caps.end()) continue;
     int mb = 0;
     FW_TRY(build_stage_blocks(c, cap, &mb));
     const size_t smem = fw::subsolve_staged_smem_bytes(p.max_interior, mb, cap, fp32, false);
-    if (smem > 227 * 1024) continue;
+    if (smem > fw::subsolve_staged_smem_max(false)) continue;
     c->stage_caps.push_back(cap);
-    if (fw::subsolve_staged_smem_bytes(p.max_interior, mb, cap, fp32, true) <= 227 * 1024)
-      c->stage_ahead_caps.push_back(cap);
     smem_max = std::max(smem_max, smem);
+    const size_t ahead = fw::subsolve_staged_smem_bytes(p.max_interior, mb, cap, fp32, true);
+    if (ahead > fw::subsolve_staged_smem_max(true)) continue;
+    c->stage_ahead_caps.push_back(cap);
+    ahead_max = std::max(ahead_max, ahead);
   }
-  c->warp_ok = !c->stage_caps.empty() && fw::configure_subsolve_staged(smem_max, fp32) == 0;
+  c->warp_ok = !c->stage_caps.empty() && fw::configure_subsolve_staged(smem_max, fp32, false) == 0;
+  if (ahead_max > 0 && fw::configure_subsolve_staged(ahead_max, fp32, true) != 0) c->stage_ahead_caps.clear();
   if (c->warp_ok) {
     // the default: the middle capacity
     FW_TRY(build_stage_blocks(c, c->stage_caps[(c->stage_caps.size() - 1) / 2 + (c->stage_caps.size() > 2 ? 1 : 0)],

@@ -1140,6 +1140,10 @@ __device__ bool staged_backward_ahead(Stage<T> &st, int nblk, const int2 *rows_g
   return true;
 }
 
+constexpr int kPlainWarps = 4;  // most warps of the plain sweeps
+constexpr int kAheadWarps = 8;  // and of those that take rows ahead
+constexpr size_t sweep_static_smem(int warps) { return (size_t)warps * 2 * sizeof(double); }
+
 // kAhead: 0 for the plain sweeps with one, two or four warps, otherwise the
 // number of warps of the sweeps that take the rows ahead.
 template <typename T, bool kInv, int kAhead>
@@ -1149,8 +1153,8 @@ __global__ void __launch_bounds__(kAhead ? 32 * kAhead : 128)
   if (mode == kModeIter && p.sc->status != 0) return;
   if (accumulate && refine_skipped(p, mode)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  constexpr int kMaxWarps = kAhead ? kAhead : 4;
-  __shared__ double red[kMaxWarps][2];
+  constexpr int kMaxWarps = kAhead ? kAhead : kPlainWarps;
+  __shared__ double red[kMaxWarps][2];  // sweep_static_smem
   const int nt = kAhead ? 32 * kAhead : blockDim.x, nw = nt >> 5;
   const int tid = threadIdx.x;
   const int s = p.sub_order[blockIdx.x];
@@ -1995,27 +1999,31 @@ int raise_smem_limit(const void *func, int slot, size_t smem) {
   return 0;
 }
 
+// A CTA's 227 KB less the sweep's static part
+size_t subsolve_staged_smem_max(bool ahead) {
+  return 227 * 1024 - sweep_static_smem(ahead ? kAheadWarps : kPlainWarps);
+}
+
 namespace {
+// The plain sweep, or the two that take rows ahead.  They are configured by
+// themselves: the latter hold two more row tables and more static memory, and
+// where only the plain one fits it has to run all the same.
 template <typename T, bool kInv>
-int configure_sweep(int slot, size_t smem) {
-  const void *const f[kSweepVariants] = {(const void *)subsolve_staged_kernel<T, kInv, 0>,
-                                         (const void *)subsolve_staged_kernel<T, kInv, 4>,
-                                         (const void *)subsolve_staged_kernel<T, kInv, 8>};
-  if (smem > 227 * 1024) return -1;
-  // the sweeps that take rows ahead hold two more row tables
-  const size_t ahead = std::min<size_t>(smem + 2 * kSB * 8, 227 * 1024);
-  for (int k = 0; k < kSweepVariants; k++)
-    if (const int rc = raise_smem_limit(f[k], slot + k, k == 0 ? smem : ahead)) return rc;
-  return 0;
+int configure_sweep(int slot, size_t smem, bool ahead) {
+  if (!ahead) return raise_smem_limit((const void *)subsolve_staged_kernel<T, kInv, 0>, slot, smem);
+  if (const int rc = raise_smem_limit((const void *)subsolve_staged_kernel<T, kInv, 4>, slot + 1, smem)) return rc;
+  return raise_smem_limit((const void *)subsolve_staged_kernel<T, kInv, kAheadWarps>, slot + 2, smem);
 }
 }  // namespace
 
-int configure_subsolve_staged(size_t smem, bool fp32) {
-  return fp32 ? configure_sweep<float2, false>(kSlotStaged32, smem) : configure_sweep<double2, false>(kSlotStaged64, smem);
+int configure_subsolve_staged(size_t smem, bool fp32, bool ahead) {
+  return fp32 ? configure_sweep<float2, false>(kSlotStaged32, smem, ahead)
+              : configure_sweep<double2, false>(kSlotStaged64, smem, ahead);
 }
 
-int configure_subsolve_inv(size_t smem, bool fp32) {
-  return fp32 ? configure_sweep<float2, true>(kSlotInv32, smem) : configure_sweep<double2, true>(kSlotInv64, smem);
+int configure_subsolve_inv(size_t smem, bool fp32, bool ahead) {
+  return fp32 ? configure_sweep<float2, true>(kSlotInv32, smem, ahead)
+              : configure_sweep<double2, true>(kSlotInv64, smem, ahead);
 }
 
 void launch_row_table(const DevProblem &p, const int64_t *ptr, int2 *tab, cudaStream_t stream) {

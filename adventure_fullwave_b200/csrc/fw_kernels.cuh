@@ -204,8 +204,9 @@ void launch_subsolve(const DevProblem &p, int mode, bool fp32, cudaStream_t stre
 size_t subsolve_smem_bytes(int max_interior, int max_iface, bool fp32);
 int configure_subsolve(size_t smem, bool fp32);
 size_t subsolve_staged_smem_bytes(int max_interior, int max_blocks, int cap, bool fp32, bool ahead);
-int configure_subsolve_staged(size_t smem, bool fp32);
-int configure_subsolve_inv(size_t smem, bool fp32);
+size_t subsolve_staged_smem_max(bool ahead);  // most that a CTA may take
+int configure_subsolve_staged(size_t smem, bool fp32, bool ahead);
+int configure_subsolve_inv(size_t smem, bool fp32, bool ahead);
 // the block-inverse layout (DevProblem inv_*) from the FP64 factor L64 in the
 // envelope layout, in FP32 (Linv32) or FP64 (Linv64)
 void launch_row_table(const DevProblem &p, const int64_t *ptr, int2 *tab, cudaStream_t stream);
