@@ -28,6 +28,7 @@ NOALLOC_MAX_ROWS = 262144
 PREC_FP64 = 0
 PREC_FP32_IR = 1
 MAX_RHS = 16
+HOOK_ALLOC_MAX = 0
 
 c_i32 = ctypes.c_int32
 c_i64 = ctypes.c_int64
@@ -148,6 +149,7 @@ SIGNATURES = {
     "fwgpu_get_skyline_profile": [ctypes.c_void_p, c_i32, P(c_i32), P(c_i32), P(c_i32)],
     "fwgpu_get_tmp_aij": [ctypes.c_void_p, c_i32, P(c_i32), P(c_i32), P(c_i32), P(c_dbl), P(c_dbl)],
     "fwgpu_get_factor": [ctypes.c_void_p, c_i32, P(c_dbl)],
+    "fwgpu_test_hook": [ctypes.c_void_p, c_i32, c_i64],
 }
 
 

@@ -58,6 +58,7 @@ struct fwgpu_context {
   fwgpu_options opts{};
   cudaStream_t stream = nullptr;
   std::vector<void *> allocs;
+  int64_t alloc_max = 0;  // test hook: larger allocations fail (0: off)
   int stage = 0;  // 0 created, 1 assembled, 2 first solve, 3 interface iteration, 4 last step
 
   // static device data
@@ -74,6 +75,7 @@ struct fwgpu_context {
   std::vector<int64_t> h_env_ptr;
   int64_t nlen_int = 0;
   int64_t nlen_ref = 0;
+  bool layout_ok = false;          // build_layout is done
   double2 *d_L64 = nullptr;
   float2 *d_L32 = nullptr;
   int32_t *d_env_lo = nullptr;
@@ -165,9 +167,12 @@ struct fwgpu_context {
     *ptr = nullptr;
     if (count == 0) count = 1;
     void *raw = nullptr;
-    cudaError_t e = cudaMalloc(&raw, count * sizeof(T));
-    if (e != cudaSuccess)
+    cudaError_t e = cudaErrorMemoryAllocation;
+    if (alloc_max <= 0 || count * sizeof(T) <= (size_t)alloc_max) e = cudaMalloc(&raw, count * sizeof(T));
+    if (e != cudaSuccess) {
+      (void)cudaGetLastError();  // or a repeated call's check of its launches reports it
       return set_error(FWGPU_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+    }
     allocs.push_back(raw);
     *ptr = (T *)raw;
     return FWGPU_OK;
@@ -905,6 +910,13 @@ int fwgpu_get_sizes(const fwgpu_context *c, fwgpu_sizes *sz) {
   return FWGPU_OK;
 }
 
+int fwgpu_test_hook(fwgpu_context *c, int32_t hook, int64_t value) {
+  if (!c) return set_error(FWGPU_ERR_ARG, "null context");
+  if (hook != FWGPU_HOOK_ALLOC_MAX || value < 0) return set_error(FWGPU_ERR_ARG, "unknown test hook or value");
+  c->alloc_max = value;
+  return FWGPU_OK;
+}
+
 int fwgpu_set_element_source(fwgpu_context *c, const fwgpu_element_source *es) {
   if (c && c->cojo_flag >= 0) return set_error(FWGPU_ERR_STATE, "a correction-Jo context solves only fwgpu_cojo_solve");
   if (!c) return set_error(FWGPU_ERR_ARG, "null context");
@@ -1032,7 +1044,7 @@ static int build_row_table(fwgpu_context *c, const int64_t *d_ptr, const int2 **
 // (the rows' entries left of the block, the block's N = (I + L_bb)^-1 - I as
 // a dense strict lower triangle, and its pivots) fit one staging buffer of
 // `cap` elements, each subdomain's elements from a 16-byte boundary.
-static int build_inv_blocks(fwgpu_context *c, int cap, bool optional) {
+static int build_inv_blocks(fwgpu_context *c, int cap) {
   const fw::Plan &p = c->p;
   const int nsub = c->m.nsub;
   const bool fp32 = c->opts.precision == FWGPU_PREC_FP32_IR;
@@ -1083,12 +1095,12 @@ static int build_inv_blocks(fwgpu_context *c, int cap, bool optional) {
     return FWGPU_OK;
   }
   // padding: bulk copies of a block may read up to 16 bytes past its end
+  // no room for it is an error, not the staged sweep: that one sums in another
+  // order, and the solution would depend on the memory left
   const int rc = fp32 ? c->alloc(&c->d_Linv32, pos + 64) : c->alloc(&c->d_Linv64, pos + 64);
-  if (rc != FWGPU_OK && optional) {  // no room for the copy: the staged sweep
-    (void)cudaGetLastError();
-    return FWGPU_OK;
-  }
-  FW_TRY(rc);
+  if (rc != FWGPU_OK)
+    return set_error(rc, "no device memory for the block-inverse copy of the factor (the WARP solve kernel needs none): " +
+                             g_last_error);
   FW_TRY(c->upload(&c->d_inv_blk_off, boff));
   FW_TRY(c->upload(&c->d_inv_blk_tab, btab));
   FW_TRY(c->upload(&c->d_inv_ptr, iptr));
@@ -1245,6 +1257,81 @@ static int tune_solve_kernel(fwgpu_context *c) {
   return FWGPU_OK;
 }
 
+// The first solve's layouts: the interior envelope, the staged sweep's blocks
+// and the block-inverse copy, all fixed by the model.
+static int build_layout(fwgpu_context *c) {
+  const fw::Plan &p = c->p;
+  const int nsub = c->m.nsub;
+  const int64_t ndof = p.sub_dof_off[nsub];
+  // skyline profile on the device, envelope layout on the host
+  FW_TRY(c->alloc(&c->d_idx1, ndof));
+  c->launches += 1;
+  fw::launch_profile(nsub, c->d_dof_off, c->d_nnz_off, c->d_row_ptr, c->d_col, c->d_aval, c->d_isbc, c->d_idx1,
+                     c->stream);
+  c->h_idx1.resize(ndof);
+  FW_CUDA(cudaMemcpyAsync(c->h_idx1.data(), c->d_idx1, ndof * sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
+  FW_CUDA(cudaStreamSynchronize(c->stream));
+  // the interior envelope of every subdomain, laid out on all host threads
+  fw::EnvelopeLayout env;
+  fw::envelope_layout(p, c->h_idx1.data(), env);
+  c->h_env_lo.swap(env.env_lo);
+  c->h_env_ptr.swap(env.env_ptr);
+  const int64_t pos = env.nlen;
+  c->nlen_int = env.nlen;
+  c->nlen_ref = env.nlen_ref;
+  FW_TRY(c->upload(&c->d_env_lo, c->h_env_lo));
+  FW_TRY(c->upload(&c->d_env_ptr, c->h_env_ptr));
+  FW_TRY(c->upload(&c->d_env_dst, env.dst));
+  // padding: bulk copies of a block may read up to 16 bytes past its end
+  FW_TRY(c->alloc(&c->d_L64, pos + 64));
+  c->dp.env_lo = c->d_env_lo;
+  c->dp.env_ptr = c->d_env_ptr;
+  FW_TRY(build_row_table(c, c->d_env_ptr, &c->dp.row_tab));
+  if (c->opts.precision == FWGPU_PREC_FP32_IR) FW_TRY(c->alloc(&c->d_L32, pos + 64));
+  FW_TRY(setup_stage(c));
+  if (c->opts.solve_kernel == FWGPU_SOLVE_WARP && !c->warp_ok)
+    return set_error(FWGPU_ERR_ARG, "staged solve kernel: subdomains too large for shared memory");
+  // the block-inverse layout: asked for, or AUTO with FP32 factors, or AUTO
+  // with FP64 factors up to 1 GiB.  The triangles' chains are what few
+  // subdomains wait for, and with many its blocks of more rows save: per iteration, staged and so, 59
+  // subdomains of up to 600 elements FP64 125 and 81 us, 58 of up to 1200 318
+  // and 165, 1463 of up to 1200 758 and 644, 3811 of up to 200 177 and 166,
+  // 1654 of up to 600 277 and 268.  Above, the staged sweep: 5093 of up to
+  // 900 (1.8 GB) took 1394 and 1337, for a second copy of the factor and, on
+  // 350 iterations, a solution that moved by 2e-10 with the rounding.
+  const bool fp32 = c->opts.precision == FWGPU_PREC_FP32_IR;
+  const bool any = c->opts.solve_kernel == FWGPU_SOLVE_AUTO;
+  const bool asked = c->opts.solve_kernel == FWGPU_SOLVE_BLOCKINV;
+  constexpr int64_t kInvCopyMax = (int64_t)1 << 30;  // bytes of FP64 factor
+  if (c->warp_ok && (asked || (any && (fp32 || pos * (int64_t)sizeof(double2) <= kInvCopyMax)))) {
+    const int cap = c->opts.stage_cap <= 0 ? inv_stage_cap(c) : any && !fp32 ? c->dp.stage_cap : c->opts.stage_cap;
+    FW_TRY(build_inv_blocks(c, cap));
+  }
+  if (c->opts.solve_kernel == FWGPU_SOLVE_BLOCKINV && !c->inv_ok)
+    return set_error(FWGPU_ERR_ARG, "block-inverse solve kernel: subdomains too large for shared memory");
+  c->layout_ok = true;
+  return FWGPU_OK;
+}
+
+// What a build_layout that failed half-way had made (every allocation after
+// the first `mark`), so that the next call builds the same again and never
+// runs on a part of it.
+static void drop_layout(fwgpu_context *c, size_t mark) {
+  (void)cudaStreamSynchronize(c->stream);
+  while (c->allocs.size() > mark) {
+    cudaFree(c->allocs.back());
+    c->allocs.pop_back();
+  }
+  c->d_idx1 = c->d_env_lo = c->d_blk_off = c->d_inv_blk_off = nullptr;
+  c->d_env_ptr = c->d_env_dst = c->d_inv_ptr = nullptr;
+  c->d_blk_tab = c->d_inv_blk_tab = nullptr;
+  c->d_L64 = c->d_Linv64 = nullptr;
+  c->d_L32 = c->d_Linv32 = nullptr;
+  c->stage_caps.clear();
+  c->stage_ahead_caps.clear();
+  c->warp_ok = c->inv_ok = c->inv_ahead_ok = false;
+}
+
 int fwgpu_solve_dom_1st(fwgpu_context *c) {
   Trace trace("solve_dom_1st");
   if (!c) return set_error(FWGPU_ERR_ARG, "null context");
@@ -1252,55 +1339,13 @@ int fwgpu_solve_dom_1st(fwgpu_context *c) {
   FW_CUDA(cudaSetDevice(c->opts.device));
   FW_TRY(clear_copy_timeout(c));
   const fw::Plan &p = c->p;
-  const int nsub = c->m.nsub;
-  const int64_t ndof = p.sub_dof_off[nsub];
-  if (!c->d_L64) {
-    // skyline profile on the device, envelope layout on the host
-    FW_TRY(c->alloc(&c->d_idx1, ndof));
-    c->launches += 1;
-    fw::launch_profile(nsub, c->d_dof_off, c->d_nnz_off, c->d_row_ptr, c->d_col, c->d_aval, c->d_isbc, c->d_idx1,
-                       c->stream);
-    c->h_idx1.resize(ndof);
-    FW_CUDA(cudaMemcpyAsync(c->h_idx1.data(), c->d_idx1, ndof * sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
-    FW_CUDA(cudaStreamSynchronize(c->stream));
-    // the interior envelope of every subdomain, laid out on all host threads
-    fw::EnvelopeLayout env;
-    fw::envelope_layout(p, c->h_idx1.data(), env);
-    c->h_env_lo.swap(env.env_lo);
-    c->h_env_ptr.swap(env.env_ptr);
-    const int64_t pos = env.nlen;
-    c->nlen_int = env.nlen;
-    c->nlen_ref = env.nlen_ref;
-    FW_TRY(c->upload(&c->d_env_lo, c->h_env_lo));
-    FW_TRY(c->upload(&c->d_env_ptr, c->h_env_ptr));
-    FW_TRY(c->upload(&c->d_env_dst, env.dst));
-    // padding: bulk copies of a block may read up to 16 bytes past its end
-    FW_TRY(c->alloc(&c->d_L64, pos + 64));
-    c->dp.env_lo = c->d_env_lo;
-    c->dp.env_ptr = c->d_env_ptr;
-    FW_TRY(build_row_table(c, c->d_env_ptr, &c->dp.row_tab));
-    if (c->opts.precision == FWGPU_PREC_FP32_IR) FW_TRY(c->alloc(&c->d_L32, pos + 64));
-    FW_TRY(setup_stage(c));
-    if (c->opts.solve_kernel == FWGPU_SOLVE_WARP && !c->warp_ok)
-      return set_error(FWGPU_ERR_ARG, "staged solve kernel: subdomains too large for shared memory");
-    // the block-inverse layout: asked for, or AUTO with FP32 factors, or AUTO
-    // with FP64 factors up to 1 GiB.  The triangles' chains are what few
-    // subdomains wait for, and with many its blocks of more rows save: per iteration, staged and so, 59
-    // subdomains of up to 600 elements FP64 125 and 81 us, 58 of up to 1200 318
-    // and 165, 1463 of up to 1200 758 and 644, 3811 of up to 200 177 and 166,
-    // 1654 of up to 600 277 and 268.  Above, the staged sweep: 5093 of up to
-    // 900 (1.8 GB) took 1394 and 1337, for a second copy of the factor and, on
-    // 350 iterations, a solution that moved by 2e-10 with the rounding.
-    const bool fp32 = c->opts.precision == FWGPU_PREC_FP32_IR;
-    const bool any = c->opts.solve_kernel == FWGPU_SOLVE_AUTO;
-    const bool asked = c->opts.solve_kernel == FWGPU_SOLVE_BLOCKINV;
-    constexpr int64_t kInvCopyMax = (int64_t)1 << 30;  // bytes of FP64 factor
-    if (c->warp_ok && (asked || (any && (fp32 || pos * (int64_t)sizeof(double2) <= kInvCopyMax)))) {
-      const int cap = c->opts.stage_cap <= 0 ? inv_stage_cap(c) : any && !fp32 ? c->dp.stage_cap : c->opts.stage_cap;
-      FW_TRY(build_inv_blocks(c, cap, any && !fp32));
+  if (!c->layout_ok) {
+    const size_t mark = c->allocs.size();
+    const int rc = build_layout(c);
+    if (rc != FWGPU_OK) {
+      drop_layout(c, mark);
+      return rc;
     }
-    if (c->opts.solve_kernel == FWGPU_SOLVE_BLOCKINV && !c->inv_ok)
-      return set_error(FWGPU_ERR_ARG, "block-inverse solve kernel: subdomains too large for shared memory");
   }
   if (!c->factor_fresh) {
     // envelope values and LDL^T factor (the layout is fixed by the model)

@@ -545,6 +545,13 @@ int fwgpu_get_tmp_aij(fwgpu_context *ctx, int32_t s, int32_t *nnz, int32_t *row_
  * (mat[idx2[i]+j], 1/d on the diagonal); nlen complex values. */
 int fwgpu_get_factor(fwgpu_context *ctx, int32_t s, double *mat);
 
+/* -- test hooks ----------------------------------------------------------- */
+
+/* Sets one of the hooks below on a context; never needed in normal use. */
+#define FWGPU_HOOK_ALLOC_MAX 0 /* device allocations of more than `value` bytes fail as they do when
+                                  there is no room (0: off) */
+int fwgpu_test_hook(fwgpu_context *ctx, int32_t hook, int64_t value);
+
 #ifdef __cplusplus
 }
 #endif
