@@ -102,7 +102,7 @@ struct fwgpu_context {
   bool factor_fresh = false;       // factor matches the assembled values
   bool solve_tuned = false;        // the subdomain-solve kernel has been chosen
   // assembly work buffers kept for the context's lifetime (repeated solves)
-  double *d_elmat = nullptr;       // element matrices, 72 doubles per element
+  double *d_elmat = nullptr;       // element matrices, 72 doubles per element; later the block-inverse copy (inv_in_elmat)
   int64_t *d_cpl_src = nullptr, *d_ifr_src = nullptr, *d_aii_src = nullptr, *d_diag_src = nullptr;
   std::vector<int32_t> h_src_owner, h_src_local;  // first subdomain holding each edge, and its local DOF
   bool warp_ok = false;            // the staged warp-per-subdomain kernel fits in shared memory
@@ -129,6 +129,7 @@ struct fwgpu_context {
   int2 *d_inv_blk_tab = nullptr;
   double2 *d_Linv64 = nullptr;
   float2 *d_Linv32 = nullptr;
+  bool inv_in_elmat = false;       // the copy lies in d_elmat
   std::vector<int> stage_caps;     // staging capacities that fit in shared memory
   std::vector<int> stage_ahead_caps;  // those with room for the sweeps that take rows ahead
   std::vector<int32_t> h_order;    // subdomains by interior size, largest first (the device sub_order)
@@ -928,10 +929,7 @@ int fwgpu_set_element_source(fwgpu_context *c, const fwgpu_element_source *es) {
   return set_element_source(c, es);
 }
 
-int fwgpu_make_tmp_aij(fwgpu_context *c, const fwgpu_source *src) {
-  Trace trace("make_TMP_AIJ");
-  if (!c) return set_error(FWGPU_ERR_ARG, "null context");
-  FW_CUDA(cudaSetDevice(c->opts.device));
+static int assemble(fwgpu_context *c, const fwgpu_source *src) {
   const fw::Plan &p = c->p;
   FW_CUDA(cudaEventRecord(c->ev[0], c->stream));
   if (!c->d_elmat) {
@@ -966,6 +964,18 @@ int fwgpu_make_tmp_aij(fwgpu_context *c, const fwgpu_source *src) {
   c->stage = 1;
   c->factor_fresh = false;
   return FWGPU_OK;
+}
+
+int fwgpu_make_tmp_aij(fwgpu_context *c, const fwgpu_source *src) {
+  Trace trace("make_TMP_AIJ");
+  if (!c) return set_error(FWGPU_ERR_ARG, "null context");
+  FW_CUDA(cudaSetDevice(c->opts.device));
+  const int rc = assemble(c, src);
+  // a source was refused: the factors stay in use, and the element matrices
+  // may have been written over their block-inverse copy
+  if (rc != FWGPU_OK && c->inv_in_elmat && c->factor_fresh)
+    fw::launch_inv_relayout(c->dp, c->d_L64, c->opts.precision == FWGPU_PREC_FP32_IR, c->stream);
+  return rc;
 }
 
 // Row blocks of the staged solve: at most 32 rows, and stored entries that
@@ -1095,12 +1105,25 @@ static int build_inv_blocks(fwgpu_context *c, int cap) {
     return FWGPU_OK;
   }
   // padding: bulk copies of a block may read up to 16 bytes past its end
-  // no room for it is an error, not the staged sweep: that one sums in another
-  // order, and the solution would depend on the memory left
-  const int rc = fp32 ? c->alloc(&c->d_Linv32, pos + 64) : c->alloc(&c->d_Linv64, pos + 64);
-  if (rc != FWGPU_OK)
-    return set_error(rc, "no device memory for the block-inverse copy of the factor (the WARP solve kernel needs none): " +
-                             g_last_error);
+  const size_t bytes = (pos + 64) * (fp32 ? sizeof(float2) : sizeof(double2));
+  if (bytes <= p.el_order.size() * 72 * sizeof(double)) {
+    // The copy is written after the element matrices were last read, and the
+    // next ones are computed before it is written again: where it fits (FP64:
+    // subdomains of up to about 800 elements) it takes their buffer and no
+    // memory of its own.
+    c->inv_in_elmat = true;
+    if (fp32)
+      c->d_Linv32 = (float2 *)(void *)c->d_elmat;
+    else
+      c->d_Linv64 = (double2 *)(void *)c->d_elmat;
+  } else {
+    // no room for it is an error, not the staged sweep: that one sums in another
+    // order, and the solution would depend on the memory left
+    const int rc = fp32 ? c->alloc(&c->d_Linv32, pos + 64) : c->alloc(&c->d_Linv64, pos + 64);
+    if (rc != FWGPU_OK)
+      return set_error(rc, "no device memory for the block-inverse copy of the factor (the WARP solve kernel needs none): " +
+                               g_last_error);
+  }
   FW_TRY(c->upload(&c->d_inv_blk_off, boff));
   FW_TRY(c->upload(&c->d_inv_blk_tab, btab));
   FW_TRY(c->upload(&c->d_inv_ptr, iptr));
@@ -1329,7 +1352,7 @@ static void drop_layout(fwgpu_context *c, size_t mark) {
   c->d_L32 = c->d_Linv32 = nullptr;
   c->stage_caps.clear();
   c->stage_ahead_caps.clear();
-  c->warp_ok = c->inv_ok = c->inv_ahead_ok = false;
+  c->warp_ok = c->inv_ok = c->inv_ahead_ok = c->inv_in_elmat = false;
 }
 
 int fwgpu_solve_dom_1st(fwgpu_context *c) {

@@ -46,3 +46,34 @@ def test_no_room_for_the_block_inverse_copy(precision):
         with hddm.HddmSolver(model, solve_kernel="warp", **kw) as s:
             _limit(s, limit)
             assert s.solve(0).converged
+
+
+def test_the_block_inverse_copy_takes_no_memory_of_its_own():
+    """With FP64 factors of subdomains of a few hundred elements the first
+    solve allocates nothing larger than the factor itself; the copy, which
+    holds each block's triangle in full, is larger."""
+    model = _model(10, 600)
+    with hddm.HddmSolver(model, hddm_eps=1e-9, hddm_max_loop=2000) as s:
+        r = s.solve(0)
+        want, z = s.edge_solution(), s.sizes()
+    limit = max(16 * (z["nlen_interior"] + 64), 8 * z["nnz_lower"])
+    with hddm.HddmSolver(model, hddm_eps=1e-9, hddm_max_loop=2000) as s:
+        s.make_tmp_aij(0)
+        _limit(s, limit)
+        got = s.solve(0)
+        assert (got.solve_kernel, got.iterations) == ("blockinv", r.iterations)
+        assert np.array_equal(s.edge_solution(), want)
+
+
+@pytest.mark.parametrize("leaf", [110, 600])
+@pytest.mark.parametrize("precision", ["fp64", "fp32_ir"])
+def test_refused_source_leaves_the_factors_in_use(leaf, precision):
+    model = _model(8, leaf)
+    with hddm.HddmSolver(model, hddm_eps=1e-9, hddm_max_loop=2000, precision=precision) as s:
+        s.solve(0)
+        want = s.edge_solution()
+        with pytest.raises(_lib.FwgpuError) as e:
+            s.make_tmp_aij((np.array([model.n_edges]), np.array([1.0 + 0j])))
+        assert e.value.code == _lib.ERR_ARG
+        s.resolve(0)
+        assert np.array_equal(s.edge_solution(), want)
