@@ -29,6 +29,7 @@ PREC_FP64 = 0
 PREC_FP32_IR = 1
 MAX_RHS = 16
 HOOK_ALLOC_MAX = 0
+HOOK_ALLOC_FAIL = 1
 
 c_i32 = ctypes.c_int32
 c_i64 = ctypes.c_int64

@@ -58,7 +58,8 @@ struct fwgpu_context {
   fwgpu_options opts{};
   cudaStream_t stream = nullptr;
   std::vector<void *> allocs;
-  int64_t alloc_max = 0;  // test hook: larger allocations fail (0: off)
+  // test hooks: larger allocations fail, and the alloc_fail'th from now (0: off)
+  int64_t alloc_max = 0, alloc_fail = 0;
   int stage = 0;  // 0 created, 1 assembled, 2 first solve, 3 interface iteration, 4 last step
 
   // static device data
@@ -75,7 +76,9 @@ struct fwgpu_context {
   std::vector<int64_t> h_env_ptr;
   int64_t nlen_int = 0;
   int64_t nlen_ref = 0;
-  bool layout_ok = false;          // build_layout is done
+  // groups of buffers that are there (once())
+  bool assembly_ok = false, layout_ok = false, rhs_ok = false, rhs_edge_ok = false, rhs_lists_ok = false,
+       multi_ok = false;
   double2 *d_L64 = nullptr;
   float2 *d_L32 = nullptr;
   int32_t *d_env_lo = nullptr;
@@ -169,7 +172,8 @@ struct fwgpu_context {
     if (count == 0) count = 1;
     void *raw = nullptr;
     cudaError_t e = cudaErrorMemoryAllocation;
-    if (alloc_max <= 0 || count * sizeof(T) <= (size_t)alloc_max) e = cudaMalloc(&raw, count * sizeof(T));
+    const bool refuse = (alloc_max > 0 && count * sizeof(T) > (size_t)alloc_max) || (alloc_fail > 0 && --alloc_fail == 0);
+    if (!refuse) e = cudaMalloc(&raw, count * sizeof(T));
     if (e != cudaSuccess) {
       (void)cudaGetLastError();  // or a repeated call's check of its launches reports it
       return set_error(FWGPU_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
@@ -184,6 +188,26 @@ struct fwgpu_context {
     if (rc) return rc;
     if (!v.empty()) FW_CUDA(cudaMemcpyAsync(*ptr, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, stream));
     return FWGPU_OK;
+  }
+  // Runs `make` the first time, and again after a call in which it failed: what
+  // it had allocated until then is given back, so that a repeated call has all
+  // of it or none.  `make` assigns every pointer that is used later and
+  // releases nothing allocated before it.
+  template <typename F>
+  int once(bool &done, F make) {
+    if (done) return FWGPU_OK;
+    const size_t mark = allocs.size();
+    const int rc = make();
+    if (rc == FWGPU_OK) {
+      done = true;
+      return rc;
+    }
+    (void)cudaStreamSynchronize(stream);
+    while (allocs.size() > mark) {
+      cudaFree(allocs.back());
+      allocs.pop_back();
+    }
+    return rc;
   }
   void release(void *ptr) {
     if (!ptr) return;
@@ -278,10 +302,10 @@ int build_rhs(fwgpu_context *c, const fwgpu_source *src) {
   }
   c->h_points.swap(pts);
   const size_t np = c->h_points.size();
-  if (!c->d_fI) {
+  FW_TRY(c->once(c->rhs_ok, [&] {
     FW_TRY(c->alloc(&c->d_fI, nI));
-    FW_TRY(c->alloc(&c->d_fG, nG));
-  }
+    return c->alloc(&c->d_fG, nG);
+  }));
   if (np > c->points_cap) {
     c->release(c->d_points);
     c->d_points = nullptr;
@@ -291,10 +315,11 @@ int build_rhs(fwgpu_context *c, const fwgpu_source *src) {
   }
   const bool elements = c->el_src && !c->el_src_off;
   const int64_t ndof = p.sub_dof_off[nsub];
-  if (elements && !c->d_b_local) {
-    FW_TRY(c->alloc(&c->d_b_local, ndof));
-    FW_TRY(c->alloc(&c->d_b_edge, ndof));
-  }
+  if (elements)
+    FW_TRY(c->once(c->rhs_edge_ok, [&] {
+      FW_TRY(c->alloc(&c->d_b_edge, ndof));
+      return c->alloc(&c->d_b_local, ndof);
+    }));
   FW_CUDA(cudaMemsetAsync(c->d_fI, 0, nI * sizeof(double2), c->stream));
   FW_CUDA(cudaMemsetAsync(c->d_fG, 0, nG * sizeof(double2), c->stream));
   if (elements) FW_CUDA(cudaMemsetAsync(c->d_b_edge, 0, ndof * sizeof(double2), c->stream));
@@ -323,7 +348,7 @@ int build_rhs(fwgpu_context *c, const fwgpu_source *src) {
 // 6 + element DOF), elements in subdomain order, and the local DOF of every
 // interior and interface entry; built once per context.
 int build_rhs_lists(fwgpu_context *c) {
-  if (c->d_rhs_ptr) return FWGPU_OK;
+  if (c->rhs_lists_ok) return FWGPU_OK;
   const fw::Plan &p = c->p;
   const int nsub = c->m.nsub;
   const int nd = p.el_dofs;
@@ -348,12 +373,13 @@ int build_rhs_lists(fwgpu_context *c) {
     for (int64_t k = p.sub_int_off[s]; k < p.sub_int_off[s + 1]; k++) int_pos[k] = p.sub_dof_off[s] + p.int_local[k];
     for (int64_t k = p.sub_if_off[s]; k < p.sub_if_off[s + 1]; k++) if_pos[k] = p.sub_dof_off[s] + p.if_local[k];
   }
-  FW_TRY(c->upload(&c->d_rhs_ptr, ptr));
-  FW_TRY(c->upload(&c->d_rhs_src, src));
-  FW_TRY(c->upload(&c->d_int_pos, int_pos));
-  FW_TRY(c->upload(&c->d_if_pos, if_pos));
-  FW_TRY(c->alloc(&c->d_elrhs, 6 * std::max<size_t>(1, p.el_order.size())));
-  return FWGPU_OK;
+  return c->once(c->rhs_lists_ok, [&] {
+    FW_TRY(c->upload(&c->d_rhs_ptr, ptr));
+    FW_TRY(c->upload(&c->d_rhs_src, src));
+    FW_TRY(c->upload(&c->d_int_pos, int_pos));
+    FW_TRY(c->upload(&c->d_if_pos, if_pos));
+    return c->alloc(&c->d_elrhs, 6 * std::max<size_t>(1, p.el_order.size()));
+  });
 }
 
 // Element sources: the per-element right-hand side is computed once (it
@@ -913,9 +939,16 @@ int fwgpu_get_sizes(const fwgpu_context *c, fwgpu_sizes *sz) {
 
 int fwgpu_test_hook(fwgpu_context *c, int32_t hook, int64_t value) {
   if (!c) return set_error(FWGPU_ERR_ARG, "null context");
-  if (hook != FWGPU_HOOK_ALLOC_MAX || value < 0) return set_error(FWGPU_ERR_ARG, "unknown test hook or value");
-  c->alloc_max = value;
-  return FWGPU_OK;
+  if (value < 0) return set_error(FWGPU_ERR_ARG, "negative test hook value");
+  switch (hook) {
+    case FWGPU_HOOK_ALLOC_MAX:
+      c->alloc_max = value;
+      return FWGPU_OK;
+    case FWGPU_HOOK_ALLOC_FAIL:
+      c->alloc_fail = value;
+      return FWGPU_OK;
+  }
+  return set_error(FWGPU_ERR_ARG, "unknown test hook");
 }
 
 int fwgpu_set_element_source(fwgpu_context *c, const fwgpu_element_source *es) {
@@ -932,14 +965,14 @@ int fwgpu_set_element_source(fwgpu_context *c, const fwgpu_element_source *es) {
 static int assemble(fwgpu_context *c, const fwgpu_source *src) {
   const fw::Plan &p = c->p;
   FW_CUDA(cudaEventRecord(c->ev[0], c->stream));
-  if (!c->d_elmat) {
+  FW_TRY(c->once(c->assembly_ok, [&] {
     FW_TRY(c->alloc(&c->d_elmat, p.el_order.size() * 72));
     FW_TRY(c->alloc(&c->d_aval, p.nnz_total));
     FW_TRY(c->upload(&c->d_cpl_src, p.cpl_src));
     FW_TRY(c->upload(&c->d_ifr_src, p.ifr_src));
     if (c->d_aii_val) FW_TRY(c->upload(&c->d_aii_src, p.aii_src));
-    FW_TRY(c->upload(&c->d_diag_src, p.if_diag_src));
-  }
+    return c->upload(&c->d_diag_src, p.if_diag_src);
+  }));
   c->launches += 2;
   if (c->cojo_flag >= 0)
     fw::launch_cojo_element_matrices((int64_t)p.el_order.size(), c->d_el_order, c->d_tv, c->d_crd, c->d_elmat,
@@ -1023,12 +1056,18 @@ static int build_stage_blocks(fwgpu_context *c, int cap, int *max_blocks_out) {
     c->h_nblk[s] = nb;
   }
   boff[nsub] = (int32_t)btab.size();
+  // the table in use is given back once the new one is there
+  int32_t *d_off = nullptr;
+  int2 *d_tab = nullptr;
+  FW_TRY(c->upload(&d_off, boff));
+  if (const int rc = c->upload(&d_tab, btab)) {
+    c->release(d_off);
+    return rc;
+  }
   c->release(c->d_blk_off);
   c->release(c->d_blk_tab);
-  c->d_blk_off = nullptr;
-  c->d_blk_tab = nullptr;
-  FW_TRY(c->upload(&c->d_blk_off, boff));
-  FW_TRY(c->upload(&c->d_blk_tab, btab));
+  c->d_blk_off = d_off;
+  c->d_blk_tab = d_tab;
   c->dp.blk_off = c->d_blk_off;
   c->dp.blk_tab = c->d_blk_tab;
   c->dp.max_blocks = max_blocks;
@@ -1281,11 +1320,16 @@ static int tune_solve_kernel(fwgpu_context *c) {
 }
 
 // The first solve's layouts: the interior envelope, the staged sweep's blocks
-// and the block-inverse copy, all fixed by the model.
+// and the block-inverse copy, all fixed by the model.  Run through once():
+// a repeated call never goes on with a part of them.
 static int build_layout(fwgpu_context *c) {
   const fw::Plan &p = c->p;
   const int nsub = c->m.nsub;
   const int64_t ndof = p.sub_dof_off[nsub];
+  // (a build that failed before may have left these)
+  c->d_blk_off = nullptr;
+  c->d_blk_tab = nullptr;
+  c->warp_ok = c->inv_ok = c->inv_ahead_ok = c->inv_in_elmat = false;
   // skyline profile on the device, envelope layout on the host
   FW_TRY(c->alloc(&c->d_idx1, ndof));
   c->launches += 1;
@@ -1332,27 +1376,7 @@ static int build_layout(fwgpu_context *c) {
   }
   if (c->opts.solve_kernel == FWGPU_SOLVE_BLOCKINV && !c->inv_ok)
     return set_error(FWGPU_ERR_ARG, "block-inverse solve kernel: subdomains too large for shared memory");
-  c->layout_ok = true;
   return FWGPU_OK;
-}
-
-// What a build_layout that failed half-way had made (every allocation after
-// the first `mark`), so that the next call builds the same again and never
-// runs on a part of it.
-static void drop_layout(fwgpu_context *c, size_t mark) {
-  (void)cudaStreamSynchronize(c->stream);
-  while (c->allocs.size() > mark) {
-    cudaFree(c->allocs.back());
-    c->allocs.pop_back();
-  }
-  c->d_idx1 = c->d_env_lo = c->d_blk_off = c->d_inv_blk_off = nullptr;
-  c->d_env_ptr = c->d_env_dst = c->d_inv_ptr = nullptr;
-  c->d_blk_tab = c->d_inv_blk_tab = nullptr;
-  c->d_L64 = c->d_Linv64 = nullptr;
-  c->d_L32 = c->d_Linv32 = nullptr;
-  c->stage_caps.clear();
-  c->stage_ahead_caps.clear();
-  c->warp_ok = c->inv_ok = c->inv_ahead_ok = c->inv_in_elmat = false;
 }
 
 int fwgpu_solve_dom_1st(fwgpu_context *c) {
@@ -1362,14 +1386,7 @@ int fwgpu_solve_dom_1st(fwgpu_context *c) {
   FW_CUDA(cudaSetDevice(c->opts.device));
   FW_TRY(clear_copy_timeout(c));
   const fw::Plan &p = c->p;
-  if (!c->layout_ok) {
-    const size_t mark = c->allocs.size();
-    const int rc = build_layout(c);
-    if (rc != FWGPU_OK) {
-      drop_layout(c, mark);
-      return rc;
-    }
-  }
+  FW_TRY(c->once(c->layout_ok, [&] { return build_layout(c); }));
   if (!c->factor_fresh) {
     // envelope values and LDL^T factor (the layout is fixed by the model)
     const int64_t pos = c->nlen_int;
@@ -1441,7 +1458,6 @@ int fwgpu_iteration_s(fwgpu_context *c, int32_t *status) {
 
 // Buffers of the batched-source solve, allocated on first use.
 static int multi_setup(fwgpu_context *c) {
-  if (c->mp.ms) return FWGPU_OK;
   const bool fp32 = c->opts.precision == FWGPU_PREC_FP32_IR;
   const fw::DevProblem &dp = c->dp;
   const int64_t R = fw::kMaxRhs;
@@ -1525,7 +1541,7 @@ static int multi_run(fwgpu_context *c, int32_t n_src, const fwgpu_source *srcs, 
   if (fw::configure_multi(smem, fp32) != 0)
     return set_error(FWGPU_ERR_ARG, "batched sources: subdomains too large for shared memory");
   set_multi_buckets(c);
-  FW_TRY(multi_setup(c));
+  FW_TRY(c->once(c->multi_ok, [&] { return multi_setup(c); }));
   fw::MultiProblem &m = c->mp;
   m.p = c->dp;
   // right-hand sides: column k of [row][kMaxRhs] is source k (the others zero)

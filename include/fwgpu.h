@@ -550,6 +550,7 @@ int fwgpu_get_factor(fwgpu_context *ctx, int32_t s, double *mat);
 /* Sets one of the hooks below on a context; never needed in normal use. */
 #define FWGPU_HOOK_ALLOC_MAX 0 /* device allocations of more than `value` bytes fail as they do when
                                   there is no room (0: off) */
+#define FWGPU_HOOK_ALLOC_FAIL 1 /* the `value`th device allocation from now fails in the same way (0: off) */
 int fwgpu_test_hook(fwgpu_context *ctx, int32_t hook, int64_t value);
 
 #ifdef __cplusplus

@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 
 from adventure_fullwave_b200 import _lib, hddm, meshgen
+from helpers import golden, rel_l2
 
 pytestmark = pytest.mark.gpu
 
@@ -77,3 +78,41 @@ def test_refused_source_leaves_the_factors_in_use(leaf, precision):
         assert e.value.code == _lib.ERR_ARG
         s.resolve(0)
         assert np.array_equal(s.edge_solution(), want)
+
+
+@pytest.mark.parametrize("precision,kernel", [("fp64", "auto"), ("fp64", "warp"), ("fp32_ir", "auto")])
+def test_every_failed_allocation_can_be_repeated(precision, kernel):
+    """Each device allocation of an element source, a solve and a batched
+    solve fails once; the failed call is an error and its repetition gives what
+    a context that always had the memory gives: AUTO the same bits, WARP, whose
+    timed staging capacity sets the order of its sums, the solution that
+    converged to 1e-10."""
+    _, _, model = golden("gap")
+    es, model.element_source = model.element_source, None
+    src = (np.array([3, 17], np.int32), np.array([1.0 + 2j, -0.5j]))
+
+    def run(fail):
+        failed = 0
+        with hddm.HddmSolver(model, hddm_eps=1e-10, hddm_max_loop=20000, precision=precision, solve_kernel=kernel) as s:
+            _lib.check(s._lib.fwgpu_test_hook(s._h, _lib.HOOK_ALLOC_FAIL, fail))
+            for call in (lambda: s.set_element_source(es), lambda: s.solve(src), lambda: s.solve_multi([src, src])):
+                try:
+                    call()
+                except _lib.FwgpuError as e:
+                    assert e.code == _lib.ERR_NOMEM
+                    failed += 1
+                    call()
+            xs = [s.edge_solution_multi(0), s.edge_solution_multi(1)]
+            s.resolve(src)
+            return [s.edge_solution(), *xs], failed
+
+    want, failed = run(0)
+    assert failed == 0
+    for k in range(1, 200):
+        got, failed = run(k)
+        for a, b in zip(got, want):
+            assert np.array_equal(a, b) if kernel == "auto" else rel_l2(a, b) <= 1e-7
+        if failed == 0:
+            break
+        assert failed == 1
+    assert k > 30  # every allocation was met
