@@ -30,6 +30,8 @@ PREC_FP32_IR = 1
 MAX_RHS = 16
 HOOK_ALLOC_MAX = 0
 HOOK_ALLOC_FAIL = 1
+HOOK_SWEEP = 2
+HOOK_ROW_FACTOR = 3
 
 c_i32 = ctypes.c_int32
 c_i64 = ctypes.c_int64
@@ -88,7 +90,7 @@ class FwResult(ctypes.Structure):
         ("iterations", c_i32), ("converged", c_i32), ("initial_norm", c_dbl), ("final_resi", c_dbl),
         ("final_resi_l2", c_dbl), ("t_setup_ms", c_dbl), ("t_iterate_ms", c_dbl), ("t_last_ms", c_dbl),
         ("kernel_launches", c_i64), ("solve_kernel", c_i32), ("stage_cap", c_i32),
-        ("stage_warps", c_i32), ("reserved", c_i32),
+        ("stage_warps", c_i32), ("stage_ahead", c_i32),
     ]
 
 

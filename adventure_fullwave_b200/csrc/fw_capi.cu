@@ -60,6 +60,9 @@ struct fwgpu_context {
   std::vector<void *> allocs;
   // test hooks: larger allocations fail, and the alloc_fail'th from now (0: off)
   int64_t alloc_max = 0, alloc_fail = 0;
+  // and the sweep's warps + 16 with rows taken ahead (0: timed), the factor row by row
+  int forced_sweep = 0;
+  bool row_factor = false;
   int stage = 0;  // 0 created, 1 assembled, 2 first solve, 3 interface iteration, 4 last step
 
   // static device data
@@ -947,8 +950,16 @@ int fwgpu_test_hook(fwgpu_context *c, int32_t hook, int64_t value) {
     case FWGPU_HOOK_ALLOC_FAIL:
       c->alloc_fail = value;
       return FWGPU_OK;
+    case FWGPU_HOOK_SWEEP:
+      if (value != 0 && value != 1 && value != 2 && value != 4 && value != 16 + 4 && value != 16 + 8) break;
+      if (c->solve_tuned) return set_error(FWGPU_ERR_STATE, "the sweep is chosen by the first solve");
+      c->forced_sweep = (int)value;
+      return FWGPU_OK;
+    case FWGPU_HOOK_ROW_FACTOR:
+      c->row_factor = value != 0;
+      return FWGPU_OK;
   }
-  return set_error(FWGPU_ERR_ARG, "unknown test hook");
+  return set_error(FWGPU_ERR_ARG, "unknown test hook or value");
 }
 
 int fwgpu_set_element_source(fwgpu_context *c, const fwgpu_element_source *es) {
@@ -1277,7 +1288,8 @@ static int tune_solve_kernel(fwgpu_context *c) {
                                                            cap) != c->stage_ahead_caps.end();
     for (int warps = 1; warps <= 8; warps *= 2)
       for (int ahead = warps == 8 ? 1 : 0; ahead <= (warps >= 4 && room ? 1 : 0); ahead++)
-        if (c->opts.stage_warps == warps || (c->opts.stage_warps == 0 && !(any && warps == 1)))
+        if (c->forced_sweep != 0 ? c->forced_sweep == warps + 16 * ahead
+                                 : c->opts.stage_warps == warps || (c->opts.stage_warps == 0 && !(any && warps == 1)))
           cand.push_back({variant, cap, warps, ahead});
   };
   // AUTO runs the block-inverse sweep where it built that layout
@@ -1395,7 +1407,8 @@ int fwgpu_solve_dom_1st(fwgpu_context *c) {
     fw::launch_scatter_envelope(p.nnz_total, c->d_env_dst, c->d_aval, c->d_L64, c->stream);
     c->dp.L64 = c->d_L64;
     FW_CUDA(cudaMemsetAsync(c->d_mesh_status + 1, 0, sizeof(int32_t), c->stream));
-    fw::launch_factor(c->dp, c->dp.int_off, c->d_env_lo, c->d_env_ptr, c->d_L64, c->d_mesh_status + 1, c->stream);
+    fw::launch_factor(c->dp, c->dp.int_off, c->d_env_lo, c->d_env_ptr, c->d_L64, c->d_mesh_status + 1, c->row_factor,
+                      c->stream);
     FW_CUDA(cudaGetLastError());
     if (c->opts.precision == FWGPU_PREC_FP32_IR) {
       fw::launch_to_fp32(pos + 64, c->d_L64, c->d_L32, c->stream);
@@ -1603,7 +1616,7 @@ static int multi_run(fwgpu_context *c, int32_t n_src, const fwgpu_source *srcs, 
     res[k].solve_kernel = fw::kSolveWarp + 1;
     res[k].stage_cap = c->dp.stage_cap;
     res[k].stage_warps = c->dp.stage_warps;
-    res[k].reserved = 0;
+    res[k].stage_ahead = 0;
     all_conv &= sc.converged;
     any_bad |= sc.nonfinite;
   }
@@ -1937,7 +1950,7 @@ static int fill_result(fwgpu_context *c, fwgpu_result *res) {
                                                             : 0;
     res->stage_warps =
         c->dp.solve_variant == fw::kSolveWarp || c->dp.solve_variant == fw::kSolveInv ? c->dp.stage_warps : 0;
-    res->reserved = 0;
+    res->stage_ahead = res->stage_warps > 0 ? c->dp.stage_ahead : 0;
   }
   if (sc.nonfinite) return set_error(FWGPU_ERR_NONFINITE, "the interface residual became NaN or infinite");
   return sc.converged ? FWGPU_OK : set_error(FWGPU_ERR_NOT_CONVERGED, "hddm_max_loop reached before hddm_eps");

@@ -1884,7 +1884,7 @@ void launch_diag_pc(int64_t n, const int64_t *diag_src, const double2 *aval, dou
 }
 
 void launch_factor(const DevProblem &p, const int64_t *int_off, const int32_t *env_lo, const int64_t *env_ptr,
-                   double2 *L, int32_t *status, cudaStream_t stream) {
+                   double2 *L, int32_t *status, bool by_rows, cudaStream_t stream) {
   if (p.nsub <= 0) return;
   // one CTA per subdomain while its row table fits in shared memory (9,600
   // interior DOFs).  The rows below a block are shared by the CTA's eight-lane
@@ -1899,7 +1899,7 @@ void launch_factor(const DevProblem &p, const int64_t *int_off, const int32_t *e
                                     : factor_block_kernel<256>;
   const int threads = per_sm <= 2 ? 1024 : per_sm <= 4 ? 512 : 256;
   const int slot = per_sm <= 2 ? kSlotFactor1024 : per_sm <= 4 ? kSlotFactor512 : kSlotFactor;
-  if (raise_smem_limit((const void *)kernel, slot, smem) == 0) {
+  if (!by_rows && raise_smem_limit((const void *)kernel, slot, smem) == 0) {
     kernel<<<p.nsub, threads, smem, stream>>>(p.sub_order, int_off, env_lo, env_ptr, L, status);
     return;
   }

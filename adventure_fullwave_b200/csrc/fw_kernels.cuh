@@ -197,8 +197,9 @@ void launch_profile(int32_t nsub, const int64_t *dof_off, const int64_t *nnz_off
 void launch_scatter_envelope(int64_t nnz, const int64_t *dst, const double2 *aval, double2 *L, cudaStream_t stream);
 void launch_gather_ops(int64_t n, const int64_t *src, const double2 *aval, double2 *dst, cudaStream_t stream);
 void launch_diag_pc(int64_t n, const int64_t *diag_src, const double2 *aval, double2 *pcloc, cudaStream_t stream);
+// by_rows: the kernel of the largest subdomains whatever the size (same bits)
 void launch_factor(const DevProblem &p, const int64_t *int_off, const int32_t *env_lo, const int64_t *env_ptr,
-                   double2 *L, int32_t *status, cudaStream_t stream);
+                   double2 *L, int32_t *status, bool by_rows, cudaStream_t stream);
 void launch_to_fp32(int64_t n, const double2 *src, float2 *dst, cudaStream_t stream);
 void launch_subsolve(const DevProblem &p, int mode, bool fp32, cudaStream_t stream);
 size_t subsolve_smem_bytes(int max_interior, int max_iface, bool fp32);

@@ -51,6 +51,7 @@ class HddmResult:
     solve_kernel: str = ""
     stage_cap: int = 0
     stage_warps: int = 0
+    stage_ahead: int = 0
 
 
 def _mesh_struct(model):
@@ -284,7 +285,7 @@ class HddmSolver:
         return HddmResult(int(r.iterations), bool(r.converged), float(r.initial_norm), float(r.final_resi),
                           float(r.final_resi_l2), float(r.t_setup_ms), float(r.t_iterate_ms), float(r.t_last_ms),
                           int(r.kernel_launches), _KERNEL_NAMES.get(int(r.solve_kernel), ""),
-                          int(r.stage_cap), int(r.stage_warps))
+                          int(r.stage_cap), int(r.stage_warps), int(r.stage_ahead))
 
     def adjoint_gradient(self, probe_edges=None, design_tets=None):
         """Backward of the last ``solve``: J = sum |x_p|^2 over ``probe_edges``

@@ -199,7 +199,7 @@ typedef struct {
   int32_t solve_kernel;    /* FWGPU_SOLVE_* used for the subdomain solves */
   int32_t stage_cap;       /* WARP kernel: envelope elements per staging buffer, else 0 */
   int32_t stage_warps;     /* WARP kernel: warps per subdomain, else 0 */
-  int32_t reserved;
+  int32_t stage_ahead;     /* 1: these warps take the next block's rows ahead of the block's end, else 0 */
 } fwgpu_result;
 
 /* -- lifecycle ----------------------------------------------------------- */
@@ -551,6 +551,11 @@ int fwgpu_get_factor(fwgpu_context *ctx, int32_t s, double *mat);
 #define FWGPU_HOOK_ALLOC_MAX 0 /* device allocations of more than `value` bytes fail as they do when
                                   there is no room (0: off) */
 #define FWGPU_HOOK_ALLOC_FAIL 1 /* the `value`th device allocation from now fails in the same way (0: off) */
+#define FWGPU_HOOK_SWEEP 2      /* before the first solve: the WARP and BLOCKINV kernels run with `value` = 1, 2 or 4
+                                   warps per subdomain, or 16 + 4 or 16 + 8: four or eight that take the next
+                                   block's rows ahead (0: timed, the same bits) */
+#define FWGPU_HOOK_ROW_FACTOR 3 /* 1: factors by the kernel for subdomains of over 9,600 interior DOFs
+                                   (0: by size, the same bits) */
 int fwgpu_test_hook(fwgpu_context *ctx, int32_t hook, int64_t value);
 
 #ifdef __cplusplus
