@@ -26,9 +26,8 @@ __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
   return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
 // a b with its roundings spelled out (re: a.x b.x fused, im: a.y b.x fused):
-// where a kernel must give the bits of another one, both of its products are
-// in this form or in the one with a and b exchanged, whichever contraction
-// the compiler chose there, and no surrounding code can change it.
+// where a kernel must give the bits of another one, both have their products
+// in this form, and no surrounding code can change it.
 __device__ __forceinline__ double2 cmul_rn(double2 a, double2 b) {
   return make_double2(__fma_rn(a.x, b.x, -__dmul_rn(a.y, b.y)), __fma_rn(a.y, b.x, __dmul_rn(a.x, b.y)));
 }

@@ -144,7 +144,8 @@ __global__ void to_fp32_kernel(int64_t n, const double2 *__restrict__ src, float
 // row-Crout without pivoting, in place: off-diagonals become L (unit lower),
 // the diagonal becomes 1/d.  The dot product of each (i, j) step is split
 // over 32 partial sums, k = k0 + l, k0 + l + 32, ..., which a butterfly adds
-// up; both kernels below sum in this order and give the same bits.
+// up; both kernels below sum in this order, with products whose roundings are
+// spelled out, and give the same bits.
 //
 // One warp per subdomain, row by row: any size.
 __global__ void factor_kernel(int32_t nsub, const int32_t *__restrict__ sub_order, const int64_t *__restrict__ int_off,
@@ -167,7 +168,7 @@ __global__ void factor_kernel(int32_t nsub, const int32_t *__restrict__ sub_orde
       const double2 *Lj = L + ptr[j] - lo_j;
       const int k0 = lo_i > lo_j ? lo_i : lo_j;
       double2 acc = cz();
-      for (int k = k0 + lane; k < j; k += 32) acc = cadd(acc, cmul(Gi[k], Lj[k]));
+      for (int k = k0 + lane; k < j; k += 32) acc = cadd(acc, cmul_rn(Gi[k], Lj[k]));
       acc = warp_sum(acc);
       if (lane == 0) Gi[j] = csub(Gi[j], acc);
       __syncwarp();
@@ -176,8 +177,8 @@ __global__ void factor_kernel(int32_t nsub, const int32_t *__restrict__ sub_orde
     for (int k = lo_i + lane; k < i; k += 32) {
       const double2 g = Gi[k];
       const double2 dk = L[ptr[k] + (k - lo[k])];
-      acc = cadd(acc, cmul(cmul(g, g), dk));
-      Gi[k] = cmul(g, dk);
+      acc = cadd(acc, cmul_rn(cmul_rn(g, g), dk));
+      Gi[k] = cmul_rn(g, dk);
     }
     acc = warp_sum(acc);
     if (lane == 0) {
