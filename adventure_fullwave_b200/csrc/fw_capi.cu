@@ -1615,7 +1615,7 @@ static int multi_run(fwgpu_context *c, int32_t n_src, const fwgpu_source *srcs, 
     res[k].kernel_launches = c->launches;
     res[k].solve_kernel = fw::kSolveWarp + 1;
     res[k].stage_cap = c->dp.stage_cap;
-    res[k].stage_warps = c->dp.stage_warps;
+    res[k].stage_warps = fw::kMultiSweepWarps;
     res[k].stage_ahead = 0;
     all_conv &= sc.converged;
     any_bad |= sc.nonfinite;

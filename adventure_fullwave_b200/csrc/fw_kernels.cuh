@@ -168,6 +168,7 @@ struct MultiProblem {
 };
 
 size_t multi_smem_bytes(int max_interior, int max_blocks, int cap, bool fp32);
+constexpr int kMultiSweepWarps = 8;  // of one CTA: a subdomain, eight of the sources
 int multi_ctas_per_sm(size_t smem);  // sweep CTAs that fit one SM (at most 2: registers)
 int configure_multi(size_t smem, bool fp32);
 void launch_multi_subsolve(const MultiProblem &m, int mode, bool fp32, cudaStream_t stream);

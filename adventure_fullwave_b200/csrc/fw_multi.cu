@@ -132,7 +132,7 @@ __global__ void multi_residual_kernel(MultiProblem m, int mode) {
 // ---- the sweeps --------------------------------------------------------------
 
 constexpr int kRS = 8;             // sources of one CTA
-constexpr int kSweepThreads = 256; // 32 rows (or columns) x kRS sources at a time
+constexpr int kSweepThreads = 32 * kMultiSweepWarps;  // 32 rows (or columns) x kRS sources at a time
 
 struct MultiLayout {
   size_t y, buf0, buf1, dinv, meta, rect, bar, blk, total;

@@ -139,15 +139,17 @@ typedef struct {
                             ir_tol * |rhs| (0 = always ir_max_steps) */
   int32_t graph_iterations; /* COCG iterations captured per CUDA graph launch */
   int32_t device;        /* CUDA device ordinal */
-  int32_t solve_kernel;  /* FWGPU_SOLVE_*: batched subdomain-solve kernel (0 = timed choice) */
-  int32_t stage_cap;     /* WARP kernel: envelope elements per staging buffer (0 = timed choice) */
+  int32_t solve_kernel;  /* FWGPU_SOLVE_*: batched subdomain-solve kernel (0 = AUTO) */
+  int32_t stage_cap;     /* WARP and BLOCKINV kernels: factor elements per staging buffer (0 = a rule on the
+                            model; WARP asked for by name: timed) */
   double ir_relax;       /* FP32_IR: interface iterations refine only while the COCG relative
                             residual is above ir_relax (0 = always); the first and last
                             subdomain solves always refine */
   int32_t shard_begin;   /* sharded solve: this context solves subdomains [shard_begin, shard_end) */
   int32_t shard_end;     /* (0, 0 = every subdomain, unsharded); a given range, even all of them,
                             makes a sharded context: drive it with the fwgpu_shard_* calls */
-  int32_t stage_warps;   /* WARP kernel: warps sharing a subdomain's sweeps, 1, 2 or 4 (0 = timed choice) */
+  int32_t stage_warps;   /* WARP and BLOCKINV kernels: warps sharing a subdomain's sweeps, 1, 2 or 4 (4: with the
+                            next block's rows taken ahead or not, timed; 0 = timed choice, which may be 8) */
   int32_t stall_copy_test; /* test hook, 0 in normal use: 1 makes the staged subdomain solves' first wait
                               for a copy poll a barrier that nothing completes, give up after a few polls
                               and raise FWGPU_ERR_TIMEOUT (each CTA still waits for its copies in flight
@@ -160,7 +162,7 @@ typedef struct {
  * sum in the same order; WARP also times its staging capacities, which
  * changes the order of the sums. */
 #define FWGPU_SOLVE_AUTO 0
-#define FWGPU_SOLVE_WARP 1   /* one warp per subdomain, vectors in shared memory */
+#define FWGPU_SOLVE_WARP 1   /* one CTA of one to eight warps per subdomain, vectors in shared memory */
 #define FWGPU_SOLVE_CTA 2    /* one 256-thread CTA per subdomain */
 #define FWGPU_SOLVE_GLOBAL 3 /* one warp per subdomain, vectors in global memory (any size) */
 #define FWGPU_SOLVE_BLOCKINV 4 /* the WARP kernel on a second layout of the factor: each row block's own
@@ -197,8 +199,9 @@ typedef struct {
   double t_last_ms;        /* final subdomain solves, device time */
   int64_t kernel_launches; /* kernels this library launched for the call */
   int32_t solve_kernel;    /* FWGPU_SOLVE_* used for the subdomain solves */
-  int32_t stage_cap;       /* WARP kernel: envelope elements per staging buffer, else 0 */
-  int32_t stage_warps;     /* WARP kernel: warps per subdomain, else 0 */
+  int32_t stage_cap;       /* WARP and BLOCKINV kernels: factor elements per staging buffer, else 0 */
+  int32_t stage_warps;     /* WARP and BLOCKINV kernels: warps per subdomain (1, 2, 4 or 8), else 0; batched
+                              sources: 8, for every eight of the 16 sources */
   int32_t stage_ahead;     /* 1: these warps take the next block's rows ahead of the block's end, else 0 */
 } fwgpu_result;
 

@@ -54,3 +54,15 @@ def test_same_bits_of_both_factor_kernels(n, leaf):
             s.solve_dom_1st()
             got.append([s.factor(k) for k in range(model.nsub)])
     assert all(np.array_equal(a, b) for a, b in zip(*got))
+
+
+@pytest.mark.parametrize("warps", [0, 1])
+def test_batched_result_names_its_own_sweep(warps):
+    """Batched sources run eight warps, whatever the one-source sweep was
+    given or timed to."""
+    model = _model(5, 30)
+    with hddm.HddmSolver(model, hddm_eps=1e-9, hddm_max_loop=2000, stage_warps=warps) as s:
+        r, = s.solve_multi([0])
+        assert (r.solve_kernel, r.stage_warps, r.stage_ahead) == ("warp", 8, 0)
+        one = s.resolve(0)
+        assert one.stage_warps == warps if warps else one.stage_warps > 1
