@@ -32,6 +32,7 @@ HOOK_ALLOC_MAX = 0
 HOOK_ALLOC_FAIL = 1
 HOOK_SWEEP = 2
 HOOK_ROW_FACTOR = 3
+HOOK_COPY_MAX = 4
 
 c_i32 = ctypes.c_int32
 c_i64 = ctypes.c_int64

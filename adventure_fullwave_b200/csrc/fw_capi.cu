@@ -63,6 +63,8 @@ struct fwgpu_context {
   // and the sweep's warps + 16 with rows taken ahead (0: timed), the factor row by row
   int forced_sweep = 0;
   bool row_factor = false;
+  // FP64 AUTO: bytes of factor up to which the block-inverse copy may take memory of its own
+  int64_t inv_own_max = (int64_t)1 << 30;
   int stage = 0;  // 0 created, 1 assembled, 2 first solve, 3 interface iteration, 4 last step
 
   // static device data
@@ -955,6 +957,10 @@ int fwgpu_test_hook(fwgpu_context *c, int32_t hook, int64_t value) {
       if (c->solve_tuned) return set_error(FWGPU_ERR_STATE, "the sweep is chosen by the first solve");
       c->forced_sweep = (int)value;
       return FWGPU_OK;
+    case FWGPU_HOOK_COPY_MAX:
+      if (value == 0) break;
+      c->inv_own_max = value;
+      return FWGPU_OK;
     case FWGPU_HOOK_ROW_FACTOR:
       c->row_factor = value != 0;
       return FWGPU_OK;
@@ -1104,7 +1110,9 @@ static int build_row_table(fwgpu_context *c, const int64_t *d_ptr, const int2 **
 // (the rows' entries left of the block, the block's N = (I + L_bb)^-1 - I as
 // a dense strict lower triangle, and its pivots) fit one staging buffer of
 // `cap` elements, each subdomain's elements from a 16-byte boundary.
-static int build_inv_blocks(fwgpu_context *c, int cap) {
+// own_max: the factor's bytes up to which the copy may take memory of its own
+// (0: any); beyond, without room in the element matrices, there is no copy.
+static int build_inv_blocks(fwgpu_context *c, int cap, int64_t own_max) {
   const fw::Plan &p = c->p;
   const int nsub = c->m.nsub;
   const bool fp32 = c->opts.precision == FWGPU_PREC_FP32_IR;
@@ -1156,7 +1164,9 @@ static int build_inv_blocks(fwgpu_context *c, int cap) {
   }
   // padding: bulk copies of a block may read up to 16 bytes past its end
   const size_t bytes = (pos + 64) * (fp32 ? sizeof(float2) : sizeof(double2));
-  if (bytes <= p.el_order.size() * 72 * sizeof(double)) {
+  const bool fits = bytes <= p.el_order.size() * 72 * sizeof(double);
+  if (!fits && own_max > 0 && c->nlen_int * (int64_t)sizeof(double2) > own_max) return FWGPU_OK;
+  if (fits) {
     // The copy is written after the element matrices were last read, and the
     // next ones are computed before it is written again: where it fits (FP64:
     // subdomains of up to about 800 elements) it takes their buffer and no
@@ -1240,8 +1250,17 @@ static int setup_stage(fwgpu_context *c) {
 //     with 3072 (one).
 //   - More, FP64, 22 rows: 1463 of up to 1200 743 us with 1024, 613 with
 //     1536, 659 with 2048; 1654 of up to 600 244 with 1024, 252 with 1536;
-//     3811 of up to 200 141 and 155.  FP32 keeps the staged kernel's: 2253 of
-//     up to 1000 take 849, 814, 812 and 829 us with 1536, 2048, 2560, 3072.
+//     3811 of up to 200 141 and 155; 985 of up to 200 49 with both.  FP32 keeps
+//     the staged kernel's 2048: 2253 of up to 1000 take 849, 814, 812 and 829 us
+//     with 1536, 2048, 2560, 3072; 1654 of up to 600 328, 322 and 335 with 1536,
+//     2048, 3072; 2163 of up to 900 701, 672, 680; 1463 of up to 1200 921, 793,
+//     787; 2877 of up to 200 132 with 1024 and 153.
+// Between the two, at seven to nine per SM, the best capacity falls with the
+// subdomains' number, and the line is lower than it need be: FP64 with 1024,
+// 1536, 2048, 2560, 897 of up to 600 (seven per SM) 202, 167, 153, 173, 1179
+// (eight) 208, 193, 188, 215; 932 of up to 1200 (seven) 707, 493, 439, 416, 1120
+// (eight) 597, 490, 514, 486, 1243 (nine) 635, 522, 559, 531.  FP32 with 2048 and
+// 4096: 1022 of up to 600 (seven) 220 and 255, 932 of up to 1200 673 and 522.
 static int inv_stage_cap(const fwgpu_context *c) {
   const bool fp32 = c->opts.precision == FWGPU_PREC_FP32_IR;
   const int64_t rows = c->p.sub_int_off[c->m.nsub];
@@ -1371,20 +1390,27 @@ static int build_layout(fwgpu_context *c) {
   if (c->opts.solve_kernel == FWGPU_SOLVE_WARP && !c->warp_ok)
     return set_error(FWGPU_ERR_ARG, "staged solve kernel: subdomains too large for shared memory");
   // the block-inverse layout: asked for, or AUTO with FP32 factors, or AUTO
-  // with FP64 factors up to 1 GiB.  The triangles' chains are what few
-  // subdomains wait for, and with many its blocks of more rows save: per iteration, staged and so, 59
-  // subdomains of up to 600 elements FP64 125 and 81 us, 58 of up to 1200 318
-  // and 165, 1463 of up to 1200 758 and 644, 3811 of up to 200 177 and 166,
-  // 1654 of up to 600 277 and 268.  Above, the staged sweep: 5093 of up to
-  // 900 (1.8 GB) took 1394 and 1337, for a second copy of the factor and, on
-  // 350 iterations, a solution that moved by 2e-10 with the rounding.
+  // with FP64 factors where its copy costs no memory (it lies in the element
+  // matrices) or up to 1 GiB of factor.  The triangles' chains are what few
+  // subdomains wait for: per iteration, staged and so, 59 subdomains of up to
+  // 600 elements FP64 125 and 81 us, 58 of up to 1200 318 and 165, 636 of up to
+  // 1200 522 and 318, 1463 of up to 1200 758 and 644.  With many per SM it
+  // gives 3 to 9 %, at any size: 1654 of up to 600 (0.24 GiB) 278 and 269,
+  // 3230 (0.47) 495 and 464, 7648 (1.1) 1097 and 1035; 20447 of up to 300 (0.68)
+  // 1241 and 1138; 2868 of up to 900 (0.93) 803 and 769, 3714 (1.2) 1039 and 990,
+  // 5093 (1.7) 1401 and 1343, 8822 (2.8) 2368 and 2273; 1633 of up to 1200 (0.93)
+  // 725 and 694, 2808 (1.6) 1197 and 1163, 6611 (3.8) 2741 and 2660.  The line
+  // therefore is one of memory: 3 to 5 % are worth a second factor of 1.1 GiB,
+  // under a hundredth of the card, and not one of several.
   const bool fp32 = c->opts.precision == FWGPU_PREC_FP32_IR;
   const bool any = c->opts.solve_kernel == FWGPU_SOLVE_AUTO;
   const bool asked = c->opts.solve_kernel == FWGPU_SOLVE_BLOCKINV;
-  constexpr int64_t kInvCopyMax = (int64_t)1 << 30;  // bytes of FP64 factor
-  if (c->warp_ok && (asked || (any && (fp32 || pos * (int64_t)sizeof(double2) <= kInvCopyMax)))) {
+  const int64_t own_max = any && !fp32 ? c->inv_own_max : 0;
+  // (the copy is never smaller than the factor)
+  const int64_t factor = pos * (int64_t)sizeof(double2), elmat = (int64_t)p.el_order.size() * 72 * sizeof(double);
+  if (c->warp_ok && (asked || (any && (fp32 || factor <= std::max(own_max, elmat))))) {
     const int cap = c->opts.stage_cap <= 0 ? inv_stage_cap(c) : any && !fp32 ? c->dp.stage_cap : c->opts.stage_cap;
-    FW_TRY(build_inv_blocks(c, cap));
+    FW_TRY(build_inv_blocks(c, cap, own_max));
   }
   if (c->opts.solve_kernel == FWGPU_SOLVE_BLOCKINV && !c->inv_ok)
     return set_error(FWGPU_ERR_ARG, "block-inverse solve kernel: subdomains too large for shared memory");

@@ -157,8 +157,9 @@ typedef struct {
 } fwgpu_options;
 
 /* Batched subdomain-solve kernels.  AUTO runs the BLOCKINV kernel (the WARP
- * kernel where the FP64 factor is over 1 GiB) at the staging capacity that a
- * rule on the envelope gives, and times 2, 4 and 8 warps per subdomain, which
+ * kernel where the FP64 factor is over 1 GiB and its copy does not fit in the
+ * element matrices, 576 bytes per element) at the staging capacity that a rule
+ * on the model gives, and times 2, 4 and 8 warps per subdomain, which
  * sum in the same order; WARP also times its staging capacities, which
  * changes the order of the sums. */
 #define FWGPU_SOLVE_AUTO 0
@@ -559,6 +560,7 @@ int fwgpu_get_factor(fwgpu_context *ctx, int32_t s, double *mat);
                                    block's rows ahead (0: timed, the same bits) */
 #define FWGPU_HOOK_ROW_FACTOR 3 /* 1: factors by the kernel for subdomains of over 9,600 interior DOFs
                                    (0: by size, the same bits) */
+#define FWGPU_HOOK_COPY_MAX 4   /* before the first solve: AUTO's limit of 1 GiB, in bytes */
 int fwgpu_test_hook(fwgpu_context *ctx, int32_t hook, int64_t value);
 
 #ifdef __cplusplus

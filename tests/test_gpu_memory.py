@@ -116,3 +116,21 @@ def test_every_failed_allocation_can_be_repeated(precision, kernel):
             break
         assert failed == 1
     assert k > 30  # every allocation was met
+
+
+@pytest.mark.parametrize("n,leaf,limit,kernel", [
+    (10, 600, 1, "blockinv"),          # in the element matrices: at any size
+    (8, 1600, 1, "warp"),              # memory of its own, over the limit
+    (8, 1600, 1 << 30, "blockinv"),
+])
+def test_auto_weighs_the_memory_that_the_copy_costs(n, leaf, limit, kernel):
+    model = _model(n, leaf)
+    with hddm.HddmSolver(model, hddm_eps=1e-9, hddm_max_loop=2000) as s:
+        _lib.check(s._lib.fwgpu_test_hook(s._h, _lib.HOOK_COPY_MAX, limit))
+        r = s.solve(0)
+        assert r.converged and r.solve_kernel == kernel
+    if kernel == "warp":  # and FP32 factors, and a kernel asked for, are not limited
+        for kw in (dict(precision="fp32_ir"), dict(solve_kernel="blockinv")):
+            with hddm.HddmSolver(model, hddm_eps=1e-9, hddm_max_loop=2000, **kw) as s:
+                _lib.check(s._lib.fwgpu_test_hook(s._h, _lib.HOOK_COPY_MAX, limit))
+                assert s.solve(0).solve_kernel == "blockinv"
