@@ -113,7 +113,7 @@ struct fwgpu_context {
   double *d_elmat = nullptr;       // element matrices, 72 doubles per element; later the block-inverse copy (inv_in_elmat)
   int64_t *d_cpl_src = nullptr, *d_ifr_src = nullptr, *d_aii_src = nullptr, *d_diag_src = nullptr;
   std::vector<int32_t> h_src_owner, h_src_local;  // first subdomain holding each edge, and its local DOF
-  bool warp_ok = false;            // the staged warp-per-subdomain kernel fits in shared memory
+  bool warp_ok = false;            // the staged kernel fits in shared memory
   bool sharded = false;            // solves a range of the subdomains (fwgpu_shard_* calls)
   // sharded solve: the caller's packed exchange and scalar buffers, and the
   // shard layout (held interface DOFs, owned, packed positions)
@@ -1202,9 +1202,9 @@ static int build_inv_blocks(fwgpu_context *c, int cap, int64_t own_max) {
   return FWGPU_OK;
 }
 
-// Staging capacities the staged kernel can run with (shared memory of one
-// warp <= 227 KB), the default one's block table, and the kernel's shared
-// memory limit set for the largest of them.
+// Staging capacities the staged kernel can run with (a CTA's shared memory at
+// most subsolve_staged_smem_max), the default one's block table, and the
+// kernel's shared-memory limit set for the largest of them.
 static int setup_stage(fwgpu_context *c) {
   const fw::Plan &p = c->p;
   const bool fp32 = c->opts.precision == FWGPU_PREC_FP32_IR;

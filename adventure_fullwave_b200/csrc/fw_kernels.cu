@@ -761,7 +761,7 @@ struct StageLayout {
   size_t y, buf0, buf1, rb, meta, bar, blk, total;
 };
 
-// Shared-memory slice of one subdomain warp of the staged solve.
+// Shared memory of one CTA (a subdomain) of the staged solve.
 __host__ __device__ inline StageLayout stage_layout(int max_interior, int max_blocks, int cap, bool fp32,
                                                    bool ahead) {
   const size_t es = fp32 ? 8 : 16;

@@ -92,10 +92,10 @@ struct DevProblem {
   int32_t stage_cap;             // envelope elements per staging buffer
   int32_t stage_warps;           // warps sharing one subdomain's sweeps (1, 2, 4, or 8 with stage_ahead)
   int32_t stage_ahead;           // the sweeps take the next block's rows ahead of the triangle's end (4 or 8 warps)
+  const int2 *row_tab, *inv_row_tab;  // sum nI: (first column, position in the subdomain's entries), staged sweeps
   // staged solve on the block-inverse layout (kSolveInv): per block of rows,
   // the rows' entries left of the block, then N = (I + L_bb)^-1 - I strictly
   // lower and row-major (row t at t(t-1)/2), then the block's pivots 1/d
-  const int2 *row_tab, *inv_row_tab;  // sum nI: (first column, position in the subdomain's entries), staged sweeps
   const int64_t *inv_ptr;        // sum nI: position of each row's left entries in Linv
   const double2 *Linv64;
   const float2 *Linv32;
@@ -129,9 +129,10 @@ struct DevProblem {
   double *dist_scal;
 };
 
-// Batched subdomain solve kernels: one warp per subdomain with TMA-staged row
-// blocks and grid-wide operator products, one CTA per subdomain, or one warp
-// per subdomain with the vectors in global memory (any size).
+// Batched subdomain solve kernels: one CTA of one to eight warps per subdomain
+// with TMA-staged row blocks and grid-wide operator products (on the envelope
+// or the block-inverse layout), one 256-thread CTA per subdomain, or one warp per
+// subdomain with the vectors in global memory (any size).
 enum SolveVariant { kSolveWarp = 0, kSolveCta = 1, kSolveGlobal = 2, kSolveInv = 3 };
 
 enum SolveMode { kModeFirst = 0, kModeIter = 1, kModeLast = 2 };
@@ -209,12 +210,10 @@ size_t subsolve_staged_smem_bytes(int max_interior, int max_blocks, int cap, boo
 size_t subsolve_staged_smem_max(bool ahead);  // most that a CTA may take
 int configure_subsolve_staged(size_t smem, bool fp32, bool ahead);
 int configure_subsolve_inv(size_t smem, bool fp32, bool ahead);
+void launch_row_table(const DevProblem &p, const int64_t *ptr, int2 *tab, cudaStream_t stream);
 // the block-inverse layout (DevProblem inv_*) from the FP64 factor L64 in the
 // envelope layout, in FP32 (Linv32) or FP64 (Linv64)
-void launch_row_table(const DevProblem &p, const int64_t *ptr, int2 *tab, cudaStream_t stream);
 void launch_inv_relayout(const DevProblem &p, const double2 *L64, bool fp32, cudaStream_t stream);
-// Raises (never lowers) the dynamic shared-memory limit of kernel `func` on
-// the current device; `slot` names the kernel.
 // SMs of a B200: the rules that must give the same choice on every run count with this
 constexpr int kSms = 148;
 // Slots of the process-wide dynamic shared-memory limits (raise_smem_limit):
@@ -234,6 +233,8 @@ enum SmemSlot {
   kSlotFactor1024,
   kSmemSlots
 };
+// Raises (never lowers) the dynamic shared-memory limit of kernel `func` on
+// the current device; `slot` names the kernel.
 int raise_smem_limit(const void *func, int slot, size_t smem);
 // kernels one launch_subsolve call issues
 int subsolve_launches(const DevProblem &p, bool fp32);

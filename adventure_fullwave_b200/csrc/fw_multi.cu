@@ -5,12 +5,12 @@
 // Every vector is stored right-hand-side minor, [row][kMaxRhs], so that the
 // 16 values of one DOF are one 256-byte (FP64) line.  The subdomain phase of
 // an iteration is three launches, as in the single-source staged path:
-//   multi_rhs_kernel     f_I - A_IG v for every (interior row, source),
+//   multi_rhs_kernel     f_I - A_IG v for every (interior row, two sources),
 //   multi_sweep_kernel   the envelope sweeps, one CTA per subdomain and
 //                        kRS sources; the factor entries come from the
 //                        TMA-staged row blocks as shared-memory broadcasts,
 //                        so one staged block serves kRS sources,
-//   multi_iface_kernel   q = A_G.[x; v] (- f_G) for every (slot, source).
+//   multi_iface_kernel   q = A_G.[x; v] (- f_G) for every (slot, two sources).
 // The COCG kernels keep one set of scalars and a stopping status per source
 // (ITERATION_S, hddm_solver_s.h:260-400, per source); a finished source
 // keeps its vectors while the others go on.
@@ -186,8 +186,8 @@ inline MultiLayout multi_layout(int max_interior, int max_blocks, int cap, bool 
 // The order of every sum is that of a row taken by kQ lane groups (FP64: 4,
 // FP32: 2), whatever the number of warps.  One warp for all the sources of a
 // subdomain, as before, left each row a chain of shuffles on one warp per
-// scheduler (16 sources on 551 subdomains of up to 600 elements: 1.97 ms per
-// iteration, FP32+IR on 83 of up to 1,000: 8.3 ms).
+// scheduler (16 sources on 551 subdomains of up to 600 elements: 1.96 ms per
+// iteration, 0.73 so; FP32+IR on 123 of up to 1,000: 8.26 and 0.93 ms).
 template <typename T>
 __global__ void __launch_bounds__(kSweepThreads, 2) multi_sweep_kernel(MultiProblem m, int mode, const double2 *rhs,
                                                                    double2 *xout, int accumulate, MultiLayout lay,
